@@ -3,7 +3,7 @@
 //
 //   part[s][i][c0 + c] = sum_{j in split s, j != i} G(i, j) Q(j, c)
 //   G(i, j) = n_i . (x_i - y_j) / |x_i - y_j|^3        (generated in FP32 registers)
-//   Q(j, c) = w_j p_j X[j][c0 + c]                     (packed per call)
+//   Q(j, c) = w_j p_j X[j][c0 + c]                     (packed per call, in the sorted order)
 //
 // G is the adjoint double-layer kernel of laplace3d_DT (src/kernel/laplace3d.jl:30-40);
 // the contraction replaces the batched lfmm3d(nd = K) of
@@ -363,18 +363,18 @@ __device__ __forceinline__ void tc_body(const Params& P, const int tile, const i
     const uint32_t t_sum = tmem + 2u * (uint32_t)npad;
 
     // tile origin: coordinates are rounded to FP32 relative to it
-    const int64_t io = P.g.perm[min(i0, n - 1)];
-    const double ox = P.g.x[io], oy = P.g.y[io], oz = P.g.z[io];
+    const TileInfo& ti = P.g.tiles[tile];
+    const double ox = ti.o[0], oy = ti.o[1], oz = ti.o[2];
 
     if (warp < NGEN / 32) {
         // ------------------------- generators -------------------------------
         const int r = threadIdx.x & (M - 1);  // tile row
         const int qt = threadIdx.x / M;       // which 64 / NQ sources of each chunk (warp-uniform)
-        const bool valid = i0 + r < n;
-        const int64_t i = valid ? (int64_t)P.g.perm[i0 + r] : n;  // original index of the target
+        const int64_t i = P.g.perm[i0 + r];  // the target's node, -1 in a padding slot
+        const bool valid = i >= 0;
         float xi, yi, zi, n0, n1, n2;
         if (valid) {
-            xi = (float)(P.g.x[i] - ox); yi = (float)(P.g.y[i] - oy); zi = (float)(P.g.z[i] - oz);
+            xi = (float)(P.g.sx[i0 + r] - ox); yi = (float)(P.g.sy[i0 + r] - oy); zi = (float)(P.g.sz[i0 + r] - oz);
             n0 = (float)P.g.nx[i]; n1 = (float)P.g.ny[i]; n2 = (float)P.g.nz[i];
         } else {
             xi = yi = zi = -1.0e18f;  // far from every node and every padded source: G underflows to 0
@@ -443,13 +443,13 @@ __device__ __forceinline__ void tc_body(const Params& P, const int tile, const i
             if (lc >= SA && !mbar_wait(&empty_a[s], (uint32_t)(lc / SA - 1) & 1u, abort_flag, P.wait_limit)) { ok = false; break; }
             uint8_t* As = A + s * NP * a_bytes;
             const float* cs = crd + sc * 3 * KC;
-            const bool self = (i >= j0) && (i < j0 + KC);  // this chunk holds the target's own node
+            const bool self = (i0 + r >= j0) && (i0 + r < j0 + KC);  // this chunk holds the target itself
             const int gq0 = qt * (8 / NQ);
             if (ax < 3)
-                gen_row_part<true, NP, NQ>(cs + oa, cs + ob, cs + oc, t2a, t2b, t2c, n2x, n2y, n2z, gq0, self, j0, i,
+                gen_row_part<true, NP, NQ>(cs + oa, cs + ob, cs + oc, t2a, t2b, t2c, n2x, n2y, n2z, gq0, self, j0, i0 + r,
                                            As, a_bytes, row_off, rsw);
             else
-                gen_row_part<false, NP, NQ>(cs, cs + KC, cs + 2 * KC, t2x, t2y, t2z, n2x, n2y, n2z, gq0, self, j0, i,
+                gen_row_part<false, NP, NQ>(cs, cs + KC, cs + 2 * KC, t2x, t2y, t2z, n2x, n2y, n2z, gq0, self, j0, i0 + r,
                                             As, a_bytes, row_off, rsw);
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             mbar_arrive(&full_a[s]);
@@ -500,14 +500,14 @@ __device__ __forceinline__ void tc_body(const Params& P, const int tile, const i
                 const uint64_t da = sw128_desc(smem_u32(A + s * NP * a_bytes));
                 const uint64_t db = sw128_desc(smem_u32(B + sb * NP * b_bytes));
                 const uint32_t dacc = tmem + (uint32_t)(b * npad);
-                // products of pieces whose orders sum to at most NP - 1
+                // all four products of two pieces, or the six of three whose orders sum to at most 2
 #pragma unroll
                 for (int kk = 0; kk < KC / 16; ++kk) {
                     bool first = pfirst && kk == 0;
 #pragma unroll
                     for (int pa = 0; pa < NP; ++pa)
 #pragma unroll
-                        for (int pb = 0; pb + pa < NP; ++pb) {
+                        for (int pb = 0; pb < (NP == 2 ? 2 : NP - pa); ++pb) {
                             mma_bf16(dacc, da + (uint64_t)((pa * a_bytes + kk * 32) >> 4),
                                      db + (uint64_t)((pb * b_bytes + kk * 32) >> 4), idesc, first ? 0u : 1u);
                             first = false;
@@ -549,10 +549,7 @@ __device__ __forceinline__ void tc_body(const Params& P, const int tile, const i
 #pragma unroll
             for (int h = 0; h < KC / 32; ++h) {
                 const int64_t j = j0 + lane + 32 * h;
-                x[h] = y[h] = z[h] = 1.0e18f;  // padded source: G underflows to 0
-                if (j < n) {
-                    x[h] = (float)(P.g.x[j] - ox); y[h] = (float)(P.g.y[j] - oy); z[h] = (float)(P.g.z[j] - oz);
-                }
+                x[h] = (float)(P.g.sx[j] - ox); y[h] = (float)(P.g.sy[j] - oy); z[h] = (float)(P.g.sz[j] - oz);
             }
             const int sc = c % SC;
             if (c >= SC && !mbar_wait(&crd_empty[sc], (uint32_t)(c / SC - 1) & 1u, abort_flag, P.wait_limit)) return false;
@@ -614,7 +611,7 @@ __global__ void __launch_bounds__(nthreads<NQ>(), 4 / NQ)
 
 // Packs Q(j, c) = w_j p_j X[j][c0 + c] as NP bf16 pieces, in the swizzled K-major
 // smem image of each 64-source chunk: [chunk][piece][row c][128 B]. Rows c >= keff
-// and sources j >= n are zero.
+// and padding slots are zero.
 template <int NP>
 __global__ void k_pack_q(GeomDev g, const double* __restrict__ X, int ldx, int c0, int keff,
                          const double* __restrict__ pre, int npad, int64_t nchunks, uint8_t* __restrict__ out) {
@@ -630,7 +627,8 @@ __global__ void k_pack_q(GeomDev g, const double* __restrict__ X, int ldx, int c
     for (int q = 0; q < 8; ++q) {
         const int64_t j = ch * KC + gq * 8 + q;
         double val = 0.0;
-        if (j < g.n && c < keff) val = g.w[j] * (pre ? pre[j] : 1.0) * X[j * ldx + c0 + c];
+        const int64_t p = g.perm[j];
+        if (p >= 0 && c < keff) val = g.sw[j] * (pre ? pre[p] : 1.0) * X[p * ldx + c0 + c];
         v[q] = (float)val;
     }
     uint32_t w[4][NP];
@@ -704,7 +702,7 @@ template <int NP>
 void pack_q(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, uint8_t* bpack,
             cudaStream_t s) {
     const int npad = ((kc + 15) / 16) * 16;
-    const int64_t nchunks = (g.n + KC - 1) / KC;
+    const int64_t nchunks = g.ns / KC;
     const int64_t pk = nchunks * npad * 8;
     k_pack_q<NP><<<(unsigned)((pk + 255) / 256), 256, 0, s>>>(g, X, ldx, c0, kc, pre, npad, nchunks, bpack);
     BIE_CK(cudaGetLastError());
@@ -714,7 +712,7 @@ template <int NP>
 void launch_tc(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit, int64_t cps,
                float* part, int ldp, uint8_t* bpack, int* err, int force_ctas, cudaStream_t s) {
     const int npad = ((kc + 15) / 16) * 16;
-    const int64_t nchunks = (g.n + KC - 1) / KC;
+    const int64_t nchunks = g.ns / KC;
     pack_q<NP>(g, X, ldx, c0, kc, pre, bpack, s);
     Params P;
     P.g = g;
@@ -734,7 +732,7 @@ void launch_tc(const GeomDev& g, const double* X, int ldx, int c0, int kc, const
     P.ldp = ldp;
     P.c0 = c0;
     P.err = err;
-    dim3 grid((unsigned)((g.n + M - 1) / M), (unsigned)nsplit);
+    dim3 grid((unsigned)(g.ns / M), (unsigned)nsplit);
     if (sh.nq == 2)
         launch_k<NP, 2>(P, grid, sh.smem, s);
     else
@@ -759,7 +757,7 @@ void launch_tc_list(const std::vector<TcMember>& ms, int* err, void* dscratch, s
         P.bpack = t.bpack;
         P.npad = ((t.kc + 15) / 16) * 16;
         P.keff = t.kc;
-        P.nchunks = (t.g.n + KC - 1) / KC;
+        P.nchunks = t.g.ns / KC;
         P.cps = t.cps;
         P.stall_test = 0;
         P.wait_limit = kWaitLimit;
@@ -769,7 +767,7 @@ void launch_tc_list(const std::vector<TcMember>& ms, int* err, void* dscratch, s
         P.ldp = t.ldp;
         P.c0 = t.c0;
         P.err = err;
-        const int tiles = (int)((t.g.n + M - 1) / M);
+        const int tiles = (int)(t.g.ns / M);
         for (int sp = 0; sp < t.nsplit; ++sp)
             for (int ti = 0; ti < tiles; ++ti) items.push_back(make_int4((int)m, ti, sp, 0));
     }
@@ -822,9 +820,8 @@ void launch_block_tc(const GeomDev& g, const double* X, int ldx, int c0, int kc,
         tc::launch_tc<2>(g, X, ldx, c0, kc, pre, nsplit, cps, part, ldp, bpack, err, force_ctas, s);
 }
 
-size_t block_tc_pack_bytes(int64_t n, int kc, int pieces) {
-    const int64_t nchunks = (n + tc::KC - 1) / tc::KC;
-    return (size_t)nchunks * pieces * tc_npad(kc) * 128;
+size_t block_tc_pack_bytes(int64_t slots, int kc, int pieces) {
+    return (size_t)(slots / tc::KC) * pieces * tc_npad(kc) * 128;
 }
 
 int block_tc_ctas_per_sm(int kc, int pieces, int force_ctas) {

@@ -18,9 +18,9 @@ __device__ __forceinline__ float2 upk2(uint64_t r) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(r));
     return v;
 }
-__device__ __forceinline__ uint64_t sub2(uint64_t a, uint64_t b) {
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
     uint64_t d;
-    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
     return d;
 }
 __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
@@ -46,24 +46,72 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     return y;
 }
 
-// Device-resident geometry: SoA FP64 arrays of length n.
+// Tiles of kTB consecutive slots of the sorted node order (GeomDev). A planar tile's nodes
+// share one plane x_axis = const with normals +-e_axis, and that plane's nodes are the slots
+// [s0, s1): the kernel n_x . (x - y) / |x - y|^3 of such a target and such a source is exactly
+// zero, so the direct sums leave those slots out. axis = 3, s0 = s1 = 0: any other tile. o: the
+// middle of the tile's bounding box (the plane itself along a planar tile's axis), the origin
+// that the FP32 sums round coordinates relative to.
+struct TileInfo {
+    int32_t axis, s0, s1;
+    double o[3];
+};
+
+// Device-resident geometry: SoA FP64 arrays of length n in the caller's node order, and the
+// sorted order of the direct sums. Sorted order: the nodes of each coordinate plane with at
+// least kPlaneMin nodes on it (axis-aligned normals) together, the others after them, each
+// group bisected into compact tiles (coordinates rounded to FP32 relative to a tile's middle stay
+// accurate for near pairs) and padded to a multiple of kTB slots. Sorted coordinates are scaled by a power of two to an extent in [0.5, 1), the
+// weights by its square, which leaves the sums unchanged bit for bit and keeps 1 / r^3 in range
+// in FP32 whatever the unit of length. Padding slots: perm -1, far away (kFar), weight 0.
 struct GeomDev {
     const double *x, *y, *z;     // node positions
     const double *nx, *ny, *nz;  // node normals
     const double* w;             // quadrature weights
     int64_t n;
-    // Target order of the reduced-precision kernels: nodes sorted along a Morton
-    // curve, so that a 128-target tile is spatially compact and coordinates rounded
-    // to FP32 relative to the tile's first target stay accurate for near pairs.
-    const int32_t* perm;
+    const double *sx, *sy, *sz, *sw;  // sorted positions and weights (ns slots)
+    const int32_t* perm;              // node of each slot; null: slots are the nodes in order
+    const TileInfo* tiles;            // one per kTB slots; null: no planar tile
+    int64_t ns;                       // slots
 };
+constexpr double kFar = 1.0e18;
+constexpr int kPlaneMin = 256;
+
+// Slots a tile sums over (all but its own plane's) and the l-th of them (s0, s1 and l are
+// multiples of every source tile, so a source tile never straddles the gap).
+__device__ __forceinline__ int64_t live_slots(const GeomDev& g, const TileInfo& t) { return g.ns - (t.s1 - t.s0); }
+__device__ __forceinline__ int64_t live_slot(const TileInfo& t, int64_t l) { return l < t.s0 ? l : l + (t.s1 - t.s0); }
+// First live slot of source split y of nsplit (splits rounded up to kTS slots).
+__device__ __forceinline__ int64_t live_chunk(int64_t live, int nsplit) {
+    const int64_t c = (live + nsplit - 1) / nsplit;
+    return (c + kTS - 1) / kTS * kTS;
+}
+
+// FP64 seed of 1 / sqrt(x), relative error about 2^-20: one MUFU instruction (PTX
+// rsqrt.approx.ftz.f64).
+__device__ __forceinline__ double rsqrt_seed(double x) {
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return y;
+}
+// 1 / r^3 from r2 = r^2. With the seed y and e = 1 - r2 y^2, 1 / r^3 = y^3 (1 - e)^(-3/2), the
+// binomial series cut after e^2: the next term, 35/16 e^3, is below 2^-56 for |e| < 2^-19.
+// 7 FP64 operations, where 1 / sqrt to full precision and its cube take about 11.
+__device__ __forceinline__ double over_r3(double r2) {
+    const double y = rsqrt_seed(r2);
+    const double q = y * y;
+    const double e = fma(-r2, q, 1.0);
+    const double s = e * fma(e, 1.875, 1.5);
+    const double w = y * q;
+    return fma(w, s, w);
+}
 
 // K3 (blocktc.cu): tensor-core block direct sum for columns [c0, c0 + kc), kc <= 128,
 // kernel and right-hand sides split into `pieces` bf16 pieces (2 or 3).
 void launch_block_tc(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,
                      int64_t cps, float* part, int ldp, uint8_t* bpack, int* err, int pieces, int force_ctas,
                      cudaStream_t s);
-size_t block_tc_pack_bytes(int64_t n, int kc, int pieces);
+size_t block_tc_pack_bytes(int64_t slots, int kc, int pieces);
 // One geometry's share of a K3 work-list launch: columns [c0, c0 + kc) (kc <= 128) of X,
 // nsplit source splits of cps chunks, partials into part (ldp), Q images into bpack.
 struct TcMember {
@@ -87,7 +135,7 @@ int block_tc_ctas_per_sm(int kc, int pieces, int force_ctas = 0);
 int tc_npad(int kc);
 // K1 with the FP64 tensor-core contraction (dt64mma.cu), columns [c0, c0 + kc), kc <= 64.
 void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,
-                       int64_t chunk, double* part, int ldp, cudaStream_t s);
+                       double* part, int ldp, cudaStream_t s);
 constexpr int kTcTileM = 128;   // targets per tensor-core tile
 constexpr int kTcChunk = 64;    // sources per tensor-core chunk
 

@@ -2,22 +2,22 @@
 // on the FP64 tensor-core path (mma.sync m8n8k4 f64), the plain path of the
 // solver (FP64 end to end).
 //
-//   part[s][i][c0 + c] = sum_{j in split s, j != i} n_i.(x_i - y_j)/|x_i - y_j|^3 Q(j, c)
-//   Q(j, c) = w_j p_j X[j][c0 + c]
+//   part[s][i][c0 + c] = sum_{j in split s, j != i} n_i.(x_i - y_j)/|x_i - y_j|^3 w_j p_j X[j][c0 + c]
 //
 // Same operator as laplace3d_DT (src/kernel/laplace3d.jl:30-40) / lfmm3d pg=2
 // (src/kernel/laplace3d.jl:100-107); the 1/(4 pi) is applied by the combine.
 //
-// CTA = 4 warps = 64 targets; a warp owns 16 targets (MTW = 2 8-row m-tiles) and NC
-// columns (NC/8 n-tiles). Two m-tiles per warp keep the accumulators at 2 x NC
-// doubles, so three CTAs fit per SM (measured 10 % faster at NC = 64 than four m-tiles
-// per warp at two CTAs per SM; FP64 MMA and FP64 FMA share one throughput budget, and
-// more resident warps overlap the kernel-value generation with the MMAs). Per k-step of 4 sources each thread generates the four
-// FP64 kernel values of its A fragments (target = m-tile row l/4, source = l%4)
-// and loads its B fragments (source l%4, column l/4 of each n-tile) from shared
-// memory; 4 x NC/8 DMMAs follow. Box faces are axis-aligned, so a warp whose 32
-// targets share a normal axis forms n.(x - y) as the signed axis difference and
-// folds the sign into its output.
+// Bound by the FP64 pipes: FP64 MMA and FP64 FMA share one throughput budget, so a pair costs
+// NC + (kernel value) operations. CTA = 4 warps; a warp owns MTW 8-row m-tiles and NC columns
+// (NC / 8 n-tiles). Per k-step of 4 sources each thread generates the MTW FP64 kernel values of
+// its A fragments (target = m-tile row l/4, source = l%4), with the source's weight multiplied
+// in, and loads its B fragments (source l%4, column l/4 of each n-tile) from shared memory.
+// In a planar tile (TileInfo) the difference along the normal axis and its square belong to the
+// source and are formed once for the warp's MTW rows: 11 + 3 / MTW operations a value; other
+// tiles take 17. Sources of the tile's own plane are left out. Source tiles of TSRC sources
+// (coordinates, weights and rows of X, gathered through the sorted order) arrive by cp.async in
+// a ring of NST stages, one barrier a tile, so that the loads of the next tiles run beside the
+// sums of this one.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -29,52 +29,73 @@
 namespace bie {
 namespace d64 {
 
-constexpr int MTW = 2;  // m-tiles per warp
 constexpr int NTHR = 128;  // threads per CTA
-constexpr int TB = 32 * MTW;   // targets per CTA
-constexpr int TSRC = 32;  // sources per shared-memory tile
+constexpr int TSRC = 32;   // sources per shared-memory tile
+constexpr int NST = 3;     // stages of the source ring
+
+// m-tiles per warp and resident CTAs per SM: the accumulators take MTW * NC / 4 doubles a thread
+template <int NC> constexpr int mtw() { return NC <= 16 ? 4 : 2; }
+template <int NC> constexpr int occ() { return NC <= 32 ? 4 : 3; }
+// Row stride of a staged X tile (= 4 or 12 mod 16 doubles): the four k-rows a half-warp's
+// B-fragment load touches fall on distinct banks; rows stay 16-byte aligned.
+template <int NC> constexpr int ldq() { return NC + 4; }
+// A stage: a, b, c coordinates, weights, preconditioner (TSRC each) and the X rows.
+template <int NC> constexpr int stage_doubles() { return 5 * TSRC + TSRC * ldq<NC>(); }
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
     asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
                  : "+d"(d0), "+d"(d1)
                  : "d"(a), "d"(b));
 }
-
-template <int AX>
-__device__ __forceinline__ double kernel_val(double tx, double ty, double tz, double n0, double n1, double n2,
-                                             double sx, double sy, double sz) {
-    const double dx = tx - sx, dy = ty - sy, dz = tz - sz;
-    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    const double ri = rsqrt(r2);
-    double dn;
-    if (AX == 0) dn = dx;
-    else if (AX == 1) dn = dy;
-    else if (AX == 2) dn = dz;
-    else dn = fma(n0, dx, fma(n1, dy, n2 * dz));
-    return (dn * ri) * (ri * ri);
+// Asynchronous copies to shared memory; `live` false writes zeros and reads nothing.
+__device__ __forceinline__ void copy8(double* dst, const double* src, bool live) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(live ? 8 : 0)
+                 : "memory");
 }
+__device__ __forceinline__ void copy16(double* dst, const double* src, bool live) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(live ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-template <int NC, int AX>
-__device__ __forceinline__ void tile_step(const double* __restrict__ ssx, const double* __restrict__ ssy,
-                                          const double* __restrict__ ssz, const double* __restrict__ sq, int cnt,
-                                          const double (&tx)[MTW], const double (&ty)[MTW], const double (&tz)[MTW],
-                                          const double (&tn)[MTW][3], double (&acc)[MTW][NC / 8][2], int lane,
-                                          bool self, int64_t jt, const int64_t (&ti)[MTW]) {
-    constexpr int LDQ = NC + 4;
+// One source tile into the warp's accumulators. stg: the stage; cnt: its live sources; self:
+// the tile's first slot when it may hold one of the warp's own targets, else negative.
+template <int NC, bool PLANAR>
+__device__ __forceinline__ void tile_step(const double* __restrict__ stg, int cnt, double plane,
+                                          const double (&ta)[mtw<NC>()], const double (&tb)[mtw<NC>()],
+                                          const double (&tc)[mtw<NC>()], const double (&tn)[mtw<NC>()][3],
+                                          double (&acc)[mtw<NC>()][NC / 8][2], int lane, bool has_pre, int64_t self,
+                                          int64_t slot0) {
+    constexpr int MTW = mtw<NC>(), LDQ = ldq<NC>();
     const int kq = lane & 3, grp = lane >> 2;
+    const double* sq = stg + 5 * TSRC;
 #pragma unroll 2
-    for (int k0 = 0; k0 < cnt; k0 += 4) {
+    for (int k0 = 0; k0 < TSRC; k0 += 4) {
         const int j = k0 + kq;
-        const double sx = ssx[j], sy = ssy[j], sz = ssz[j];
+        const double sa = stg[j], sb = stg[TSRC + j], sc = stg[2 * TSRC + j];
+        double wj = stg[3 * TSRC + j];
+        if (has_pre) wj *= stg[4 * TSRC + j];
         double a[MTW];
+        if (PLANAR) {
+            const double da = plane - sa, da2 = da * da;
+            wj *= da;
 #pragma unroll
-        for (int mt = 0; mt < MTW; ++mt) {
-            a[mt] = kernel_val<AX>(tx[mt], ty[mt], tz[mt], tn[mt][0], tn[mt][1], tn[mt][2], sx, sy, sz);
-            if (self && jt + j == ti[mt]) a[mt] = 0.0;
-        }
-        if (j >= cnt) {
+            for (int mt = 0; mt < MTW; ++mt) {
+                const double db = tb[mt] - sb, dc = tc[mt] - sc;
+                a[mt] = over_r3(fma(db, db, fma(dc, dc, da2))) * wj;
+            }
+        } else {
 #pragma unroll
-            for (int mt = 0; mt < MTW; ++mt) a[mt] = 0.0;
+            for (int mt = 0; mt < MTW; ++mt) {
+                const double dx = ta[mt] - sa, dy = tb[mt] - sb, dz = tc[mt] - sc;
+                const double dn = fma(tn[mt][0], dx, fma(tn[mt][1], dy, tn[mt][2] * dz));
+                a[mt] = over_r3(fma(dx, dx, fma(dy, dy, dz * dz))) * (dn * wj);
+                if (j >= cnt || (self >= 0 && self + j == slot0 + mt * 8)) a[mt] = 0.0;
+            }
         }
         double b[NC / 8];
 #pragma unroll
@@ -87,84 +108,108 @@ __device__ __forceinline__ void tile_step(const double* __restrict__ ssx, const 
 }
 
 template <int NC>
-__global__ void __launch_bounds__(NTHR, 3) k_dt_f64_mma(GeomDev g, const double* __restrict__ X, int ldx, int c0,
-                                                     int kc, const double* __restrict__ pre, int64_t chunk,
-                                                     double* __restrict__ part, int ldp) {
-    // padded row of NC + 4 doubles (4 mod 16): the four k-rows a half-warp's B-fragment
-    // load touches fall on distinct banks
-    constexpr int LDQ = NC + 4;
-    __shared__ double ssx[TSRC + 4], ssy[TSRC + 4], ssz[TSRC + 4];
-    __shared__ double sq[(TSRC + 4) * LDQ];
+__global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const double* __restrict__ X, int ldx,
+                                                               int c0, int kc, const double* __restrict__ pre,
+                                                               double* __restrict__ part, int ldp) {
+    constexpr int MTW = mtw<NC>(), LDQ = ldq<NC>(), TB = 32 * MTW;
+    extern __shared__ __align__(16) double ring[];  // [NST][stage_doubles]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = lane >> 2, kq = lane & 3;
-    const int64_t i0 = (int64_t)blockIdx.x * TB;
-    const int64_t wbase = i0 + warp * 8 * MTW;
-    // the warp's 8 MTW targets: m-tile mt, row grp -> target wbase + 8 mt + grp
-    double tx[MTW], ty[MTW], tz[MTW], tn[MTW][3];
-    int64_t ti[MTW];
-    int code_min = 4, code_max = -1;
+    const int64_t t0 = (int64_t)blockIdx.x * TB;
+    const TileInfo ti = g.tiles ? g.tiles[t0 / kTB] : TileInfo{3, 0, 0, {0.0, 0.0, 0.0}};
+    // coordinate arrays, the tile's axis first
+    const double* pa = ti.axis == 1 ? g.sy : (ti.axis == 2 ? g.sz : g.sx);
+    const double* pb = ti.axis == 1 ? g.sz : (ti.axis == 2 ? g.sx : g.sy);
+    const double* pc = ti.axis == 1 ? g.sx : (ti.axis == 2 ? g.sy : g.sz);
+    // the thread's targets: m-tile mt, row grp -> slot slot0 + 8 mt
+    const int64_t slot0 = t0 + warp * 8 * MTW + grp;
+    double ta[MTW], tb[MTW], tc[MTW], tn[MTW][3];
 #pragma unroll
     for (int mt = 0; mt < MTW; ++mt) {
-        const int64_t i = wbase + mt * 8 + grp;
-        ti[mt] = i;
-        if (i < g.n) {
-            tx[mt] = g.x[i]; ty[mt] = g.y[i]; tz[mt] = g.z[i];
+        const int64_t slot = slot0 + 8 * mt;
+        const int64_t i = slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1;
+        ta[mt] = tb[mt] = tc[mt] = -kFar;  // no target: not stored
+        tn[mt][0] = tn[mt][1] = tn[mt][2] = 0.0;
+        if (i >= 0) {
+            ta[mt] = pa[slot]; tb[mt] = pb[slot]; tc[mt] = pc[slot];
             tn[mt][0] = g.nx[i]; tn[mt][1] = g.ny[i]; tn[mt][2] = g.nz[i];
-            int code = 3;
-            if (fabs(tn[mt][0]) == 1.0 && tn[mt][1] == 0.0 && tn[mt][2] == 0.0) code = 0;
-            else if (fabs(tn[mt][1]) == 1.0 && tn[mt][0] == 0.0 && tn[mt][2] == 0.0) code = 1;
-            else if (fabs(tn[mt][2]) == 1.0 && tn[mt][0] == 0.0 && tn[mt][1] == 0.0) code = 2;
-            code_min = min(code_min, code);
-            code_max = max(code_max, code);
-        } else {
-            tx[mt] = ty[mt] = tz[mt] = -1.0e150;  // far away: the kernel underflows to 0
-            tn[mt][0] = tn[mt][1] = tn[mt][2] = 0.0;
         }
     }
-    const unsigned full = 0xFFFFFFFFu;
-    code_min = __reduce_min_sync(full, code_min);
-    code_max = __reduce_max_sync(full, code_max);
-    const int ax = (code_min == code_max && code_min < 3) ? code_min : 3;
+    const double plane = pa[t0];
     double acc[MTW][NC / 8][2];
 #pragma unroll
     for (int mt = 0; mt < MTW; ++mt)
 #pragma unroll
         for (int nt = 0; nt < NC / 8; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
 
-    const int64_t j0 = (int64_t)blockIdx.y * chunk;
-    const int64_t j1 = min(g.n, j0 + chunk);
-    for (int64_t jt = j0; jt < j1; jt += TSRC) {
-        const int cnt = (int)min((int64_t)TSRC, j1 - jt);
-        __syncthreads();
-        for (int t = threadIdx.x; t < TSRC + 4; t += NTHR) {
-            const int64_t j = jt + t;
-            const bool v = t < cnt;
-            ssx[t] = v ? g.x[j] : 1.0e150;
-            ssy[t] = v ? g.y[j] : 1.0e150;
-            ssz[t] = v ? g.z[j] : 1.0e150;
+    const int64_t live = live_slots(g, ti), chunk = live_chunk(live, gridDim.y);
+    const int64_t l0 = (int64_t)blockIdx.y * chunk, l1 = min(live, l0 + chunk);
+    const int ntile = l1 > l0 ? (int)((l1 - l0 + TSRC - 1) / TSRC) : 0;
+    // 16-byte copies of X rows: c0 is a multiple of 64
+    const bool x16 = (ldx & 1) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    // node of the source tile's row 8 warp + lane % 8 (-1: none); the warp copies those 8 rows
+    auto row_node = [&](int t) -> int {
+        if (t >= ntile) return -1;
+        const int64_t j = live_slot(ti, l0 + (int64_t)t * TSRC) + 8 * warp + (lane & 7);
+        return j < g.ns ? (g.perm ? g.perm[j] : (int)j) : -1;
+    };
+    auto issue = [&](int t, int node) {
+        double* stg = ring + (t % NST) * stage_doubles<NC>();
+        const int64_t j = live_slot(ti, l0 + (int64_t)t * TSRC) + lane;
+        const double* arr = warp == 0 ? pa : (warp == 1 ? pb : (warp == 2 ? pc : g.sw));
+        copy8(stg + warp * TSRC + lane, arr + (j < g.ns ? j : 0), j < g.ns);
+        if (pre && lane < 8) copy8(stg + 4 * TSRC + 8 * warp + lane, pre + (node < 0 ? 0 : node), node >= 0);
+        double* sq = stg + 5 * TSRC + 8 * warp * LDQ;
+        if (x16) {
+#pragma unroll
+            for (int e0 = 0; e0 < 4 * NC; e0 += 32) {
+                const int e = e0 + lane, u = e / (NC / 2), cc = 2 * (e % (NC / 2));
+                const int p = __shfl_sync(0xFFFFFFFFu, node, u);
+                if (cc < kc) copy16(sq + u * LDQ + cc, X + (int64_t)(p < 0 ? 0 : p) * ldx + c0 + cc, p >= 0);
+            }
+        } else {
+#pragma unroll
+            for (int e0 = 0; e0 < 8 * NC; e0 += 32) {
+                const int e = e0 + lane, u = e / NC, cc = e % NC;
+                const int p = __shfl_sync(0xFFFFFFFFu, node, u);
+                if (cc < kc) copy8(sq + u * LDQ + cc, X + (int64_t)(p < 0 ? 0 : p) * ldx + c0 + cc, p >= 0);
+            }
         }
-        for (int e = threadIdx.x; e < TSRC * NC; e += NTHR) {
-            const int t = e / NC, c = e - t * NC;
-            const int64_t j = jt + t;
-            double q = 0.0;
-            if (t < cnt && c < kc) q = g.w[j] * (pre ? pre[j] : 1.0) * X[j * ldx + c0 + c];
-            sq[t * LDQ + c] = q;
-        }
+    };
+    // columns kc .. NC - 1 of the staged rows are never copied: zero, not what the memory held
+    if (kc < NC) {
+        for (int e = threadIdx.x; e < NST * stage_doubles<NC>(); e += NTHR) ring[e] = 0.0;
         __syncthreads();
-        const bool self = (jt < i0 + TB) && (jt + cnt > i0);
-        switch (ax) {
-            case 0: tile_step<NC, 0>(ssx, ssy, ssz, sq, cnt, tx, ty, tz, tn, acc, lane, self, jt, ti); break;
-            case 1: tile_step<NC, 1>(ssx, ssy, ssz, sq, cnt, tx, ty, tz, tn, acc, lane, self, jt, ti); break;
-            case 2: tile_step<NC, 2>(ssx, ssy, ssz, sq, cnt, tx, ty, tz, tn, acc, lane, self, jt, ti); break;
-            default: tile_step<NC, 3>(ssx, ssy, ssz, sq, cnt, tx, ty, tz, tn, acc, lane, self, jt, ti); break;
+    }
+#pragma unroll
+    for (int t = 0; t < NST - 1; ++t) {
+        if (t < ntile) issue(t, row_node(t));
+        copy_commit();
+    }
+    int next = row_node(NST - 1);
+    for (int t = 0; t < ntile; ++t) {
+        copy_wait<NST - 2>();
+        __syncthreads();  // tile t landed for all warps; stage (t - 1) % NST is free
+        if (t + NST - 1 < ntile) issue(t + NST - 1, next);
+        copy_commit();
+        next = row_node(t + NST);
+        const double* stg = ring + (t % NST) * stage_doubles<NC>();
+        const int cnt = (int)min((int64_t)TSRC, l1 - l0 - (int64_t)t * TSRC);
+        if (ti.axis < 3) {
+            tile_step<NC, true>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, pre != nullptr, -1, slot0);
+        } else {
+            const int64_t jt = live_slot(ti, l0 + (int64_t)t * TSRC);
+            const bool self = jt < t0 + TB && jt + TSRC > t0;
+            tile_step<NC, false>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, pre != nullptr, self ? jt : -1, slot0);
         }
     }
     // D fragment: (row grp, columns 2 kq, 2 kq + 1) of each (m-tile, n-tile)
 #pragma unroll
     for (int mt = 0; mt < MTW; ++mt) {
-        const int64_t i = ti[mt];
-        if (i >= g.n) continue;
-        const double sgn = ax == 0 ? tn[mt][0] : ax == 1 ? tn[mt][1] : ax == 2 ? tn[mt][2] : 1.0;
+        const int64_t slot = slot0 + 8 * mt;
+        const int64_t i = slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1;
+        if (i < 0) continue;
+        const double sgn = ti.axis == 0 ? g.nx[i] : (ti.axis == 1 ? g.ny[i] : (ti.axis == 2 ? g.nz[i] : 1.0));
         double* o = part + ((int64_t)blockIdx.y * g.n + i) * ldp + c0;
 #pragma unroll
         for (int nt = 0; nt < NC / 8; ++nt) {
@@ -175,20 +220,30 @@ __global__ void __launch_bounds__(NTHR, 3) k_dt_f64_mma(GeomDev g, const double*
     }
 }
 
+template <int NC>
+void launch(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit, double* part,
+            int ldp, cudaStream_t s) {
+    constexpr int TB = 32 * mtw<NC>();
+    const size_t sm = sizeof(double) * NST * stage_doubles<NC>();
+    ensure_smem_limit((const void*)k_dt_f64_mma<NC>, sm);
+    const dim3 grid((unsigned)((g.ns + TB - 1) / TB), (unsigned)nsplit);
+    k_dt_f64_mma<NC><<<grid, NTHR, sm, s>>>(g, X, ldx, c0, kc, pre, part, ldp);
+}
+
 }  // namespace d64
 
-// Columns [c0, c0 + kc) with kc <= 64 (NC = 8, 16, 32 or 64 columns per launch).
+// Columns [c0, c0 + kc) with kc <= 64 (NC = 8, 16, 32 or 64 columns per launch), c0 a multiple
+// of 64. The sources are split evenly into nsplit parts, each writing its own partial.
 void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,
-                       int64_t chunk, double* part, int ldp, cudaStream_t s) {
-    dim3 grid((unsigned)((g.n + d64::TB - 1) / d64::TB), (unsigned)nsplit);
+                       double* part, int ldp, cudaStream_t s) {
     if (kc > 32)
-        d64::k_dt_f64_mma<64><<<grid, d64::NTHR, 0, s>>>(g, X, ldx, c0, kc, pre, chunk, part, ldp);
+        d64::launch<64>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
     else if (kc > 16)
-        d64::k_dt_f64_mma<32><<<grid, d64::NTHR, 0, s>>>(g, X, ldx, c0, kc, pre, chunk, part, ldp);
+        d64::launch<32>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
     else if (kc > 8)
-        d64::k_dt_f64_mma<16><<<grid, d64::NTHR, 0, s>>>(g, X, ldx, c0, kc, pre, chunk, part, ldp);
+        d64::launch<16>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
     else
-        d64::k_dt_f64_mma<8><<<grid, d64::NTHR, 0, s>>>(g, X, ldx, c0, kc, pre, chunk, part, ldp);
+        d64::launch<8>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
     BIE_CK(cudaGetLastError());
 }
 

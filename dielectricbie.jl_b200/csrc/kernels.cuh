@@ -16,191 +16,210 @@
 namespace bie {
 
 // ---------------------------------------------------------------------------
-// K1: FP64 direct D^T sum ("plain").  part[s][i][c0 + c] =
-//   sum_{j in chunk s, j != i} n_i.(x_i - y_j) / |x_i - y_j|^3 * w_j * p_j * X[j][c0 + c]
+// K1: FP64 direct D^T sum ("plain"), fewer than 8 columns.  part[s][i][c0 + c] =
+//   sum_{j in split s, j != i} n_i.(x_i - y_j) / |x_i - y_j|^3 * w_j * p_j * X[j][c0 + c]
 // (the 1/(4 pi) is applied by the combine kernel). p = optional right
 // preconditioner (nullptr = 1). Replaces laplace3d_DT (src/kernel/laplace3d.jl:30-40)
 // and the lfmm3d pg=2 far field (src/kernel/laplace3d.jl:100-107).
+//
+// Bound by the FP64 pipe, so the work is counted in FP64 operations a pair. In a planar tile
+// x_a is the same for all targets: the difference along the axis is a property of the source,
+// its square is staged with it and it is multiplied into the source's value, which leaves 2
+// subtractions, 2 for r^2, 6 for 1 / r^3 and C for the sums; other tiles take 9 + 7 + C.
+// Sources of the tile's own plane are left out (TileInfo).
 // ---------------------------------------------------------------------------
 template <int C>
 __global__ void __launch_bounds__(kTB) k_dt_f64(GeomDev g, const double* __restrict__ X, int ldx, int c0,
-                                                  const double* __restrict__ pre, int64_t chunk,
-                                                  double* __restrict__ part, int ldp) {
-    extern __shared__ double sm[];
-    double* sx = sm;
-    double* sy = sx + kTS;
-    double* sz = sy + kTS;
-    double* sq = sz + kTS;  // [kTS][C]
-    const int64_t i0 = (int64_t)blockIdx.x * kTB;
-    const int64_t i = i0 + threadIdx.x;
-    const bool valid = i < g.n;
-    double xi = 0, yi = 0, zi = 0, n0 = 0, n1 = 0, n2 = 0;
+                                                  const double* __restrict__ pre, double* __restrict__ part, int ldp) {
+    extern __shared__ __align__(16) double sm[];
+    double* s0 = sm;        // planar: squared difference along the axis; else x
+    double* s1 = s0 + kTS;  // planar: the other two coordinates; else y, z
+    double* s2 = s1 + kTS;
+    double* sq = s2 + kTS;  // [kTS][C]
+    const TileInfo ti = g.tiles ? g.tiles[blockIdx.x] : TileInfo{3, 0, 0, {0.0, 0.0, 0.0}};
+    const bool planar = ti.axis < 3;
+    const int64_t t0 = (int64_t)blockIdx.x * kTB;
+    const int64_t slot = t0 + threadIdx.x;
+    const int64_t i = slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1;
+    const bool valid = i >= 0;
+    // coordinate arrays, the tile's axis first
+    const double* pa = ti.axis == 1 ? g.sy : (ti.axis == 2 ? g.sz : g.sx);
+    const double* pb = ti.axis == 1 ? g.sz : (ti.axis == 2 ? g.sx : g.sy);
+    const double* pc = ti.axis == 1 ? g.sx : (ti.axis == 2 ? g.sy : g.sz);
+    double xa = 0, xb = 0, xc = 0, n0 = 0, n1 = 0, n2 = 0;
     if (valid) {
-        xi = g.x[i]; yi = g.y[i]; zi = g.z[i];
+        xa = pa[slot]; xb = pb[slot]; xc = pc[slot];
         n0 = g.nx[i]; n1 = g.ny[i]; n2 = g.nz[i];
     }
+    const double plane = pa[t0];
     double acc[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) acc[c] = 0.0;
-    const int64_t j0 = (int64_t)blockIdx.y * chunk;
-    const int64_t j1 = min(g.n, j0 + chunk);
-    for (int64_t jt = j0; jt < j1; jt += kTS) {
-        const int cnt = (int)min((int64_t)kTS, j1 - jt);
+    const int64_t live = live_slots(g, ti), chunk = live_chunk(live, gridDim.y);
+    const int64_t l1 = min(live, ((int64_t)blockIdx.y + 1) * chunk);
+    for (int64_t l = (int64_t)blockIdx.y * chunk; l < l1; l += kTS) {
+        const int64_t jt = live_slot(ti, l);
+        const int cnt = (int)min((int64_t)kTS, l1 - l);
         __syncthreads();
-        for (int t = threadIdx.x; t < cnt; t += kTB) {
-            const int64_t j = jt + t;
-            sx[t] = g.x[j]; sy[t] = g.y[j]; sz[t] = g.z[j];
-            double wj = g.w[j] * (pre ? pre[j] : 1.0);
-            const double* xr = X + j * ldx + c0;
+        for (int t = threadIdx.x; t < kTS; t += kTB) {
+            double a = kFar, b = kFar, c = kFar, wj = 0.0;
+            int64_t p = -1;
+            if (t < cnt) {
+                const int64_t j = jt + t;
+                a = pa[j]; b = pb[j]; c = pc[j];
+                p = g.perm ? (int64_t)g.perm[j] : j;
+                if (p >= 0) wj = g.sw[j] * (pre ? pre[p] : 1.0);
+            }
+            if (planar) {
+                const double da = plane - a;
+                wj *= da;
+                a = da * da;
+            }
+            s0[t] = a; s1[t] = b; s2[t] = c;
 #pragma unroll
-            for (int c = 0; c < C; ++c) sq[t * C + c] = wj * xr[c];
+            for (int cc = 0; cc < C; ++cc) sq[t * C + cc] = p >= 0 ? wj * X[p * ldx + c0 + cc] : 0.0;
         }
         __syncthreads();
-        const bool self_tile = (jt < i0 + kTB) && (jt + cnt > i0);
-        if (!self_tile) {
+        if (planar) {
 #pragma unroll 2
-            for (int t = 0; t < cnt; ++t) {
-                double dx = xi - sx[t], dy = yi - sy[t], dz = zi - sz[t];
-                double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-                double ri = rsqrt(r2);
-                double nd = fma(n0, dx, fma(n1, dy, n2 * dz));
-                double gk = nd * (ri * ri * ri);
+            for (int t = 0; t < kTS; t += 2) {
+                const double2 a2 = *reinterpret_cast<const double2*>(s0 + t);
+                const double2 b2 = *reinterpret_cast<const double2*>(s1 + t);
+                const double2 c2 = *reinterpret_cast<const double2*>(s2 + t);
+                double v[2];
 #pragma unroll
-                for (int c = 0; c < C; ++c) acc[c] = fma(gk, sq[t * C + c], acc[c]);
+                for (int h = 0; h < 2; ++h) {
+                    const double db = xb - (h ? b2.y : b2.x), dc = xc - (h ? c2.y : c2.x);
+                    v[h] = over_r3(fma(db, db, fma(dc, dc, h ? a2.y : a2.x)));
+                }
+#pragma unroll
+                for (int c = 0; c < C; ++c) acc[c] = fma(v[1], sq[(t + 1) * C + c], fma(v[0], sq[t * C + c], acc[c]));
             }
         } else {
-            for (int t = 0; t < cnt; ++t) {
-                if (jt + t == i) continue;
-                double dx = xi - sx[t], dy = yi - sy[t], dz = zi - sz[t];
-                double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-                double ri = rsqrt(r2);
-                double nd = fma(n0, dx, fma(n1, dy, n2 * dz));
-                double gk = nd * (ri * ri * ri);
+            const bool self_tile = jt < t0 + kTB && jt + kTS > t0;
+#pragma unroll 2
+            for (int t = 0; t < kTS; ++t) {
+                const double dx = xa - s0[t], dy = xb - s1[t], dz = xc - s2[t];
+                const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                double v = over_r3(r2) * fma(n0, dx, fma(n1, dy, n2 * dz));
+                if (self_tile && jt + t == slot) v = 0.0;
 #pragma unroll
-                for (int c = 0; c < C; ++c) acc[c] = fma(gk, sq[t * C + c], acc[c]);
+                for (int c = 0; c < C; ++c) acc[c] = fma(v, sq[t * C + c], acc[c]);
             }
         }
     }
     if (valid) {
+        const double sgn = ti.axis == 0 ? n0 : (ti.axis == 1 ? n1 : (ti.axis == 2 ? n2 : 1.0));
         double* o = part + ((int64_t)blockIdx.y * g.n + i) * ldp + c0;
 #pragma unroll
-        for (int c = 0; c < C; ++c) o[c] = acc[c];
+        for (int c = 0; c < C; ++c) o[c] = sgn * acc[c];
     }
 }
 
 // ---------------------------------------------------------------------------
 // K2: FP32 direct D^T sum with FP64 tile partials ("refined" inner operator).
-// Targets are taken in the Morton order g.perm (compact tiles); coordinates are
-// shifted to the CTA's first target in FP64 before rounding to FP32 (keeps
-// near-pair differences accurate), rsqrt runs on the MUFU pipe, each
-// shared-memory tile accumulates in FP32 and is folded into FP64.
+// Coordinates are rounded to FP32 relative to the middle of the target tile (keeps near-pair
+// differences accurate), rsqrt runs on the MUFU pipe, each shared-memory tile accumulates in
+// FP32 and is folded into FP64.
+//
+// Bound by the FP32 pipe, then by the MUFU. Source pairs (t, t + 1) run as packed f32x2
+// operations. As in K1, a planar tile's difference along the axis and its square belong to the
+// source (7 operations and one MUFU a pair at C = 1, against 13 in other tiles), and sources of
+// the tile's own plane are left out.
 // ---------------------------------------------------------------------------
 template <int C>
 __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restrict__ X, int ldx, int c0,
-                                                  const double* __restrict__ pre, int64_t chunk,
-                                                  double* __restrict__ part, int ldp) {
-    // Source pairs (t, t + 1) run as packed f32x2 operations. Staged tiles are padded to
-    // kTS sources with far-away coordinates and zero values, so pairs never straddle
-    // the tile end.
+                                                  const double* __restrict__ pre, double* __restrict__ part, int ldp) {
     extern __shared__ __align__(16) float smf[];
-    float* sx = smf;
-    float* sy = sx + kTS;
-    float* sz = sy + kTS;
-    float* sq = sz + kTS;  // [C][kTS]: column c of the tile's sources, contiguous
-    const int64_t i0 = (int64_t)blockIdx.x * kTB;
-    const bool valid = i0 + threadIdx.x < g.n;
-    const int64_t i = valid ? (int64_t)g.perm[i0 + threadIdx.x] : g.n;  // original index of the target
-    const int64_t io = g.perm[min(i0, g.n - 1)];
-    const double ox = g.x[io], oy = g.y[io], oz = g.z[io];
-    float xi = -1.0e18f, yi = -1.0e18f, zi = -1.0e18f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
+    float* s0 = smf;        // planar: squared difference along the axis; else -x
+    float* s1 = s0 + kTS;   // minus the other two coordinates; else -y, -z
+    float* s2 = s1 + kTS;
+    float* sq = s2 + kTS;   // [C][kTS]: column c of the tile's sources, contiguous
+    const TileInfo& ti = g.tiles[blockIdx.x];
+    const int axis = ti.axis;
+    const bool planar = axis < 3;
+    const int64_t slot = (int64_t)blockIdx.x * kTB + threadIdx.x;
+    const int64_t i = g.perm[slot];  // the target's node, -1 in a padding slot
+    const bool valid = i >= 0;
+    // coordinate arrays, the tile's axis first
+    const double* pa = axis == 1 ? g.sy : (axis == 2 ? g.sz : g.sx);
+    const double* pb = axis == 1 ? g.sz : (axis == 2 ? g.sx : g.sy);
+    const double* pc = axis == 1 ? g.sx : (axis == 2 ? g.sy : g.sz);
+    const double oa = ti.o[axis == 1 ? 1 : (axis == 2 ? 2 : 0)], ob = ti.o[axis == 1 ? 2 : (axis == 2 ? 0 : 1)],
+                 oc = ti.o[axis == 1 ? 0 : (axis == 2 ? 1 : 2)];
+    float xa = -1.0e18f, xb = -1.0e18f, xc = -1.0e18f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
     if (valid) {
-        xi = (float)(g.x[i] - ox); yi = (float)(g.y[i] - oy); zi = (float)(g.z[i] - oz);
+        xa = (float)(pa[slot] - oa); xb = (float)(pb[slot] - ob); xc = (float)(pc[slot] - oc);
         n0 = (float)g.nx[i]; n1 = (float)g.ny[i]; n2 = (float)g.nz[i];
     }
-    // warp-uniform normal axis: n.(x - y) is then the signed axis difference, the sign
-    // applied to the output
-    int code = 3;
-    float sgn = 1.f;
-    if (fabsf(n0) == 1.f && n1 == 0.f && n2 == 0.f) { code = 0; sgn = n0; }
-    else if (fabsf(n1) == 1.f && n0 == 0.f && n2 == 0.f) { code = 1; sgn = n1; }
-    else if (fabsf(n2) == 1.f && n0 == 0.f && n1 == 0.f) { code = 2; sgn = n2; }
-    const int cmin = __reduce_min_sync(0xFFFFFFFFu, valid ? code : 4);
-    const int cmax = __reduce_max_sync(0xFFFFFFFFu, valid ? code : -1);
-    const int ax = (cmin == cmax && cmin < 3) ? cmin : 3;
-    if (ax == 3) sgn = 1.f;
-    const float tc[3] = {xi, yi, zi};
-    const int a1 = ax < 3 ? ax : 0, a2 = a1 == 2 ? 0 : a1 + 1, a3 = a2 == 2 ? 0 : a2 + 1;
-    const float* sA = a1 == 0 ? sx : (a1 == 1 ? sy : sz);
-    const float* sB = a2 == 0 ? sx : (a2 == 1 ? sy : sz);
-    const float* sC = a3 == 0 ? sx : (a3 == 1 ? sy : sz);
-    const uint64_t tA = pk2(tc[a1], tc[a1]), tB = pk2(tc[a2], tc[a2]), tCc = pk2(tc[a3], tc[a3]);
+    const uint64_t tA = pk2(xa, xa), tB = pk2(xb, xb), tCc = pk2(xc, xc);
     const uint64_t nA = pk2(n0, n0), nB = pk2(n1, n1), nC = pk2(n2, n2);
     const uint64_t tiny = pk2(1e-24f, 1e-24f);  // keeps the self pair's r^-3 finite: it contributes 0
     double acc[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) acc[c] = 0.0;
-    const int64_t j0 = (int64_t)blockIdx.y * chunk;
-    const int64_t j1 = min(g.n, j0 + chunk);
-    for (int64_t jt = j0; jt < j1; jt += kTS) {
-        const int cnt = (int)min((int64_t)kTS, j1 - jt);
-        __syncthreads();
-        for (int t = threadIdx.x; t < kTS; t += kTB) {
-            if (t < cnt) {
-                const int64_t j = jt + t;
-                sx[t] = (float)(g.x[j] - ox); sy[t] = (float)(g.y[j] - oy); sz[t] = (float)(g.z[j] - oz);
-                const double wj = g.w[j] * (pre ? pre[j] : 1.0);
-                const double* xr = X + j * ldx + c0;
+    const int64_t live = live_slots(g, ti), chunk = live_chunk(live, gridDim.y);
+    const int64_t l1 = min(live, ((int64_t)blockIdx.y + 1) * chunk);
+    for (int64_t l = (int64_t)blockIdx.y * chunk; l < l1; l += kTS) {
+        const int64_t j = live_slot(ti, l) + threadIdx.x;  // slots come in whole tiles
+        const int t = threadIdx.x;
+        const double a = pa[j], b = pb[j], cc = pc[j];
+        const int64_t p = g.perm[j];
+        double wj = p >= 0 ? g.sw[j] * (pre ? pre[p] : 1.0) : 0.0;
+        double xr[C];
 #pragma unroll
-                for (int c = 0; c < C; ++c) sq[c * kTS + t] = (float)(wj * xr[c]);
-            } else {
-                sx[t] = sy[t] = sz[t] = 1.0e18f;
-#pragma unroll
-                for (int c = 0; c < C; ++c) sq[c * kTS + t] = 0.f;
-            }
+        for (int c = 0; c < C; ++c) xr[c] = p >= 0 ? X[p * ldx + c0 + c] : 0.0;
+        float f0 = (float)(oa - a);
+        if (planar) {
+            wj *= oa - a;
+            f0 *= f0;
         }
+        __syncthreads();
+        s0[t] = f0; s1[t] = (float)(ob - b); s2[t] = (float)(oc - cc);
+#pragma unroll
+        for (int c = 0; c < C; ++c) sq[c * kTS + t] = (float)(wj * xr[c]);
         __syncthreads();
         uint64_t a2c[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) a2c[c] = 0ull;
-        const int cnt2 = (cnt + 1) & ~1;
-        if (ax < 3) {
+        if (planar) {
 #pragma unroll 4
-            for (int t = 0; t < cnt2; t += 2) {
-                const uint64_t da = sub2(tA, *reinterpret_cast<const uint64_t*>(sA + t));
-                const uint64_t db = sub2(tB, *reinterpret_cast<const uint64_t*>(sB + t));
-                const uint64_t dc = sub2(tCc, *reinterpret_cast<const uint64_t*>(sC + t));
-                const float2 r2 = upk2(fma2(da, da, fma2(db, db, fma2(dc, dc, tiny))));
+            for (int u = 0; u < kTS; u += 2) {
+                const uint64_t db = add2(tB, *reinterpret_cast<const uint64_t*>(s1 + u));
+                const uint64_t dc = add2(tCc, *reinterpret_cast<const uint64_t*>(s2 + u));
+                const float2 r2 = upk2(fma2(db, db, fma2(dc, dc, *reinterpret_cast<const uint64_t*>(s0 + u))));
                 const uint64_t ri = pk2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
-                const uint64_t gk = mul2(mul2(da, ri), mul2(ri, ri));
+                const uint64_t gk = mul2(ri, mul2(ri, ri));
 #pragma unroll
                 for (int c = 0; c < C; ++c)
-                    a2c[c] = fma2(gk, *reinterpret_cast<const uint64_t*>(sq + c * kTS + t), a2c[c]);
+                    a2c[c] = fma2(gk, *reinterpret_cast<const uint64_t*>(sq + c * kTS + u), a2c[c]);
             }
         } else {
 #pragma unroll 4
-            for (int t = 0; t < cnt2; t += 2) {
-                const uint64_t dx = sub2(tA, *reinterpret_cast<const uint64_t*>(sx + t));
-                const uint64_t dy = sub2(tB, *reinterpret_cast<const uint64_t*>(sy + t));
-                const uint64_t dz = sub2(tCc, *reinterpret_cast<const uint64_t*>(sz + t));
+            for (int u = 0; u < kTS; u += 2) {
+                const uint64_t dx = add2(tA, *reinterpret_cast<const uint64_t*>(s0 + u));
+                const uint64_t dy = add2(tB, *reinterpret_cast<const uint64_t*>(s1 + u));
+                const uint64_t dz = add2(tCc, *reinterpret_cast<const uint64_t*>(s2 + u));
                 const float2 r2 = upk2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, tiny))));
                 const uint64_t ri = pk2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
                 const uint64_t nd = fma2(nA, dx, fma2(nB, dy, mul2(nC, dz)));
                 const uint64_t gk = mul2(mul2(nd, ri), mul2(ri, ri));
 #pragma unroll
                 for (int c = 0; c < C; ++c)
-                    a2c[c] = fma2(gk, *reinterpret_cast<const uint64_t*>(sq + c * kTS + t), a2c[c]);
+                    a2c[c] = fma2(gk, *reinterpret_cast<const uint64_t*>(sq + c * kTS + u), a2c[c]);
             }
         }
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-            const float2 s2 = upk2(a2c[c]);
-            acc[c] += (double)s2.x + (double)s2.y;
+            const float2 s2v = upk2(a2c[c]);
+            acc[c] += (double)s2v.x + (double)s2v.y;
         }
     }
     if (valid) {
+        const double sgn = axis == 0 ? g.nx[i] : (axis == 1 ? g.ny[i] : (axis == 2 ? g.nz[i] : 1.0));
         double* o = part + ((int64_t)blockIdx.y * g.n + i) * ldp + c0;
 #pragma unroll
-        for (int c = 0; c < C; ++c) o[c] = (double)sgn * acc[c];
+        for (int c = 0; c < C; ++c) o[c] = sgn * acc[c];
     }
 }
 

@@ -104,7 +104,10 @@ void dt_apply_static(const double* x, const double* y, const double* z, const do
     g.nx = nx; g.ny = ny; g.nz = nz;
     g.w = w;
     g.n = n;
-    g.perm = nullptr;  // the FP64 kernel reads targets in node order
+    g.sx = x; g.sy = y; g.sz = z; g.sw = w;  // the nodes in the caller's order, no planar tiles
+    g.perm = nullptr;
+    g.tiles = nullptr;
+    g.ns = n;
 
     // columns per group and source splits, so that nsplit * n * kc fits the scratch. The
     // split count follows the regular FP64 path's base rule (about four waves of 128-target
@@ -122,7 +125,7 @@ void dt_apply_static(const double* x, const double* y, const double* z, const do
 
     for (int c0 = 0; c0 < k; c0 += kc) {
         const int kg = std::min(kc, k - c0);
-        launch_dt_f64_mma(g, X + c0, k, 0, kg, nullptr, (int)ns, chunk, scratch, kg, s);
+        launch_dt_f64_mma(g, X + c0, k, 0, kg, nullptr, (int)ns, scratch, kg, s);
         const int64_t total = n * kg;
         const unsigned blocks = (unsigned)std::min<int64_t>((total + 255) / 256, (int64_t)sms * 8);
         k_sum_splits<<<blocks, 256, 0, s>>>(scratch, (int)ns, n, kg, Y, k, c0);

@@ -29,7 +29,9 @@ struct bie_geom {
     int32_t npanels = 0, nb = 0;
     int64_t nblocks = 0;
     size_t geom_bytes = 0;
-    bie::Buf x, y, z, nx, ny, nz, w, diag, pinv, perm;
+    bie::Buf x, y, z, nx, ny, nz, w, diag, pinv;
+    bie::Buf sx, sy, sz, sw, perm, tiles;  // sorted order of the direct sums (GeomDev)
+    int64_t ns = 0;
     bie::Buf rowptr, col, val;
     // operator workspace
     bie::Buf part, small, bpack, errflag, cpart, srcpack, glist;
@@ -176,7 +178,9 @@ struct Prof {
 
 GeomDev gdev(const bie_geom* g) {
     return GeomDev{g->x.as<double>(), g->y.as<double>(), g->z.as<double>(), g->nx.as<double>(),
-                   g->ny.as<double>(), g->nz.as<double>(), g->w.as<double>(), g->n, g->perm.as<int32_t>()};
+                   g->ny.as<double>(), g->nz.as<double>(), g->w.as<double>(), g->n,
+                   g->sx.as<double>(), g->sy.as<double>(), g->sz.as<double>(), g->sw.as<double>(),
+                   g->perm.as<int32_t>(), g->tiles.as<TileInfo>(), g->ns};
 }
 
 template <class T>
@@ -188,13 +192,17 @@ void upload(bie::Buf& b, const T* src, size_t count, cudaStream_t s) {
 // --------------------------- direct-sum launchers --------------------------
 enum class Kern { DT64, DT32, POT64 };
 
+// Instances: DT64 with fewer than 8 columns (wider sums run dt64mma.cu's kernel), the others with
+// a power of two.
 template <int C>
 void* kern_ptr(Kern kind) {
-    switch (kind) {
-        case Kern::DT64: return (void*)k_dt_f64<C>;
-        case Kern::DT32: return (void*)k_dt_f32<C>;
-        default: return (void*)k_pot_f64<C>;
+    if constexpr (C < 8)
+        if (kind == Kern::DT64) return (void*)k_dt_f64<C>;
+    if constexpr ((C & (C - 1)) == 0) {
+        if (kind == Kern::DT32) return (void*)k_dt_f32<C>;
+        if (kind == Kern::POT64) return (void*)k_pot_f64<C>;
     }
+    throw Error(BIE_EUNSUPPORTED, "no direct-sum kernel of this width");
 }
 
 template <int C>
@@ -229,14 +237,14 @@ void launch_direct(Kern kind, const GeomDev& g, const double* X, int ldx, int c0
                    const double* T, int64_t M, Split sp, double* part, int ldp, cudaStream_t s) {
     size_t sm = kern_smem<C>(kind);
     kern_occ<C>(kind);  // sets the smem attribute
-    int64_t rows = kind == Kern::POT64 ? M : g.n;
+    int64_t rows = kind == Kern::POT64 ? M : g.ns;
     dim3 grid((unsigned)((rows + kTB - 1) / kTB), (unsigned)sp.nsplit);
-    if (kind == Kern::DT64)
-        k_dt_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, pre, sp.chunk, part, ldp);
-    else if (kind == Kern::DT32)
-        k_dt_f32<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, pre, sp.chunk, part, ldp);
-    else
-        k_pot_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, T, M, sp.chunk, part, ldp);
+    if constexpr (C < 8)
+        if (kind == Kern::DT64) k_dt_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, pre, part, ldp);
+    if constexpr ((C & (C - 1)) == 0) {
+        if (kind == Kern::DT32) k_dt_f32<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, pre, part, ldp);
+        if (kind == Kern::POT64) k_pot_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, T, M, sp.chunk, part, ldp);
+    }
     BIE_CK(cudaGetLastError());
 }
 
@@ -246,13 +254,20 @@ int occ_for(Kern kind, int C) {
         case 32: return kern_occ<32>(kind);
         case 16: return kern_occ<16>(kind);
         case 8: return kern_occ<8>(kind);
+        case 7: return kern_occ<7>(kind);
+        case 6: return kern_occ<6>(kind);
+        case 5: return kern_occ<5>(kind);
         case 4: return kern_occ<4>(kind);
+        case 3: return kern_occ<3>(kind);
         case 2: return kern_occ<2>(kind);
         default: return kern_occ<1>(kind);
     }
 }
 
-int pick_C(int rem) {
+// Columns of the next pass over rem remaining ones. The FP64 sum (fewer than 8 columns here) is
+// bound by its kernel values, so it takes all of them in one pass.
+int pick_C(Kern kind, int rem) {
+    if (kind == Kern::DT64 && rem < 8) return rem;
     static const int cs[] = {64, 32, 16, 8, 4, 2, 1};
     for (int c : cs)
         if (c <= rem) return c;
@@ -339,7 +354,7 @@ Split direct_sum(bie_geom* g, Kern kind, const double* X, int ldx, int k, const 
                 const int kc = std::min(64, k - c0);
                 std::unique_ptr<Prof> pf;
                 if (prof) pf.reset(new Prof(g, BIE_KERNEL_DIRECT_FP64, s, 1, npairs, npairs * kc));
-                launch_dt_f64_mma(gd, X, ldx, c0, kc, pre, sp.nsplit, sp.chunk, g->part.as<double>(), k, s);
+                launch_dt_f64_mma(gd, X, ldx, c0, kc, pre, sp.nsplit, g->part.as<double>(), k, s);
             }
         };
         // (the split model of 128-row tiles at two CTAs per SM, which gives the 64-target
@@ -364,22 +379,26 @@ Split direct_sum(bie_geom* g, Kern kind, const double* X, int ldx, int k, const 
         run(sp, true);
         return sp;
     }
-    int64_t rows = kind == Kern::POT64 ? M : g->n;
-    int Cmax = pick_C(k);
+    int64_t rows = kind == Kern::POT64 ? M : g->ns;
+    int Cmax = pick_C(kind, k);
     Split sp = choose_split(rows, g->n, g->sms, occ_for(kind, Cmax));
-    g->part.ensure(sizeof(double) * (size_t)sp.nsplit * std::max<int64_t>(rows, 1) * k);
+    g->part.ensure(sizeof(double) * (size_t)sp.nsplit * std::max<int64_t>(kind == Kern::POT64 ? M : g->n, 1) * k);
     double* part = g->part.as<double>();
     const int pkind = kind == Kern::DT64 ? BIE_KERNEL_DIRECT_FP64
                       : (kind == Kern::DT32 ? BIE_KERNEL_DIRECT_FP32 : BIE_KERNEL_OTHER);
     const double npairs = kind == Kern::POT64 ? (double)M * g->n : (double)g->n * (g->n - 1);
     for (int c0 = 0; c0 < k;) {
-        int C = pick_C(k - c0);
+        int C = pick_C(kind, k - c0);
         Prof pf(g, pkind, s, 1, npairs, npairs * C);
         switch (C) {
             case 64: launch_direct<64>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
             case 32: launch_direct<32>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
             case 16: launch_direct<16>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
             case 8: launch_direct<8>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
+            case 7: launch_direct<7>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
+            case 6: launch_direct<6>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
+            case 5: launch_direct<5>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
+            case 3: launch_direct<3>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
             case 4: launch_direct<4>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
             case 2: launch_direct<2>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
             default: launch_direct<1>(kind, gd, X, ldx, c0, pre, T, M, sp, part, k, s); break;
@@ -395,8 +414,8 @@ Split direct_sum(bie_geom* g, Kern kind, const double* X, int ldx, int k, const 
 // split adds an FP32 partial for the combine to read). force_ctas selects the CTA
 // shape (0 = default).
 Split tc_split(const bie_geom* g, int kc, int pieces, int force_ctas = 0) {
-    const int64_t tiles = (g->n + kTcTileM - 1) / kTcTileM;
-    const int64_t chunks = (g->n + kTcChunk - 1) / kTcChunk;
+    const int64_t tiles = g->ns / kTcTileM;
+    const int64_t chunks = g->ns / kTcChunk;
     const int64_t slots = (int64_t)g->sms * block_tc_ctas_per_sm(kc, pieces, force_ctas);
     const int64_t ns_min = std::min<int64_t>(chunks, std::max<int64_t>(1, (chunks + 1023) / 1024));
     const int64_t ns_max = std::min<int64_t>(chunks, std::max<int64_t>(ns_min, 16));
@@ -419,7 +438,7 @@ Split tc_split(const bie_geom* g, int kc, int pieces, int force_ctas = 0) {
 
 // K3 split with ns source splits (chunks per split rounded up).
 Split tc_split_n(const bie_geom* g, int64_t ns) {
-    const int64_t chunks = (g->n + kTcChunk - 1) / kTcChunk;
+    const int64_t chunks = g->ns / kTcChunk;
     ns = std::max<int64_t>(std::max<int64_t>(1, (chunks + 1023) / 1024), std::min(ns, chunks));
     const int64_t cps = (chunks + ns - 1) / ns;
     return Split{(int)((chunks + cps - 1) / cps), cps};
@@ -431,7 +450,7 @@ Split direct_sum_tc(bie_geom* g, const double* X, int k, const double* pre, int 
     const double npairs = (double)g->n * (g->n - 1);
     auto run = [&](const Split& sp, int ctas, bool prof) {
         g->part.ensure(sizeof(float) * (size_t)sp.nsplit * g->n * k);
-        g->bpack.ensure(block_tc_pack_bytes(g->n, kc0, pieces));
+        g->bpack.ensure(block_tc_pack_bytes(g->ns, kc0, pieces));
         for (int c0 = 0; c0 < k; c0 += 128) {
             int kc = std::min(128, k - c0);
             std::unique_ptr<Prof> pf;
@@ -1237,6 +1256,125 @@ void check_prec(int prec) {
 // ---------------------------------------------------------------------------
 // geometry lifetime
 // ---------------------------------------------------------------------------
+namespace {
+
+// The sorted order of the direct sums (GeomDev): scaled positions and weights, the node of each
+// slot, and each tile's plane and origin.
+struct SortedNodes {
+    std::vector<double> v[4];  // x, y, z, w
+    std::vector<int32_t> perm;
+    std::vector<TileInfo> tiles;
+};
+
+// Orders idx[0, m) so that consecutive runs of kTB nodes are compact boxes: recursive bisection
+// across the longest side, at a multiple of kTB nodes. A tile's own nodes stay in node order.
+void bisect_nodes(const double* pts, int32_t* idx, int64_t m) {
+    if (m > kTB) {
+        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+        for (int64_t e = 0; e < m; ++e)
+            for (int c = 0; c < 3; ++c) {
+                lo[c] = std::min(lo[c], pts[3 * (int64_t)idx[e] + c]);
+                hi[c] = std::max(hi[c], pts[3 * (int64_t)idx[e] + c]);
+            }
+        int ax = 0;
+        for (int c = 1; c < 3; ++c)
+            if (hi[c] - lo[c] > hi[ax] - lo[ax]) ax = c;
+        const int64_t half = ((m + kTB - 1) / kTB / 2) * kTB;
+        // coordinates that are no numbers compare as equal, so the order stays a valid one
+        std::nth_element(idx, idx + half, idx + m, [&](int32_t a, int32_t b) {
+            const double p = pts[3 * (int64_t)a + ax], q = pts[3 * (int64_t)b + ax];
+            return p < q || (p == q && a < b);
+        });
+        bisect_nodes(pts, idx, half);
+        bisect_nodes(pts, idx + half, m - half);
+    } else {
+        std::sort(idx, idx + m);
+    }
+}
+
+SortedNodes sort_nodes(const double* pts, const double* nrm, const double* w, int64_t n) {
+    double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (int64_t i = 0; i < n; ++i)
+        for (int c = 0; c < 3; ++c) {
+            lo[c] = std::min(lo[c], pts[3 * i + c]);
+            hi[c] = std::max(hi[c], pts[3 * i + c]);
+        }
+    const double ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 0.0});
+    // planes (axis, coordinate) of the axis-aligned normals, in the order of their first node
+    std::map<std::pair<int, double>, int> plane_id;
+    std::vector<std::pair<int, int64_t>> planes;  // axis, nodes
+    std::vector<int> of((size_t)n, -1);
+    int last = -1;  // nodes come panel by panel: the previous node's plane is the likely one
+    std::pair<int, double> last_key(-1, 0.0);
+    for (int64_t i = 0; i < n; ++i) {
+        const double* m = nrm + 3 * i;
+        const int ax = std::fabs(m[0]) == 1.0 && m[1] == 0.0 && m[2] == 0.0   ? 0
+                       : std::fabs(m[1]) == 1.0 && m[0] == 0.0 && m[2] == 0.0 ? 1
+                       : std::fabs(m[2]) == 1.0 && m[0] == 0.0 && m[1] == 0.0 ? 2
+                                                                              : 3;
+        if (ax == 3 || !std::isfinite(pts[3 * i + ax])) continue;
+        const std::pair<int, double> k(ax, pts[3 * i + ax]);
+        if (last < 0 || k != last_key) {
+            const auto it = plane_id.emplace(k, (int)planes.size()).first;
+            last = it->second;
+            last_key = k;
+            if (last == (int)planes.size()) planes.push_back({ax, 0});
+        }
+        of[i] = last;
+        ++planes[last].second;
+    }
+    // group starts, each group padded to whole tiles; the nodes of no (large enough) plane last
+    auto padded = [](int64_t m) { return (m + kTB - 1) / kTB * kTB; };
+    std::vector<int64_t> at(planes.size() + 1);
+    int64_t ns = 0, rest = n;
+    for (size_t p = 0; p < planes.size(); ++p) {
+        const int64_t m = planes[p].second >= kPlaneMin ? planes[p].second : 0;
+        at[p] = ns;
+        ns += padded(m);
+        rest -= m;
+    }
+    at.back() = ns;
+    ns += padded(rest);
+    SortedNodes so;
+    so.perm.assign((size_t)ns, -1);
+    so.tiles.assign((size_t)(ns / kTB), TileInfo{3, 0, 0, {0.0, 0.0, 0.0}});
+    for (size_t p = 0; p < planes.size(); ++p) {
+        if (planes[p].second < kPlaneMin) continue;
+        const int64_t s0 = at[p], s1 = s0 + padded(planes[p].second);
+        for (int64_t t = s0 / kTB; t < s1 / kTB; ++t)
+            so.tiles[t] = TileInfo{planes[p].first, (int32_t)s0, (int32_t)s1, {0.0, 0.0, 0.0}};
+    }
+    for (int64_t i = 0; i < n; ++i) {
+        const bool in_plane = of[i] >= 0 && planes[of[i]].second >= kPlaneMin;
+        so.perm[in_plane ? at[of[i]]++ : at.back()++] = (int32_t)i;
+    }
+    for (size_t p = 0; p < planes.size(); ++p)
+        if (planes[p].second >= kPlaneMin) bisect_nodes(pts, &so.perm[at[p] - planes[p].second], planes[p].second);
+    if (rest > 0) bisect_nodes(pts, &so.perm[at.back() - rest], rest);
+    int ex = 0;
+    if (std::isfinite(ext) && ext > 0.0) std::frexp(ext, &ex);
+    const double scale = std::ldexp(1.0, -std::max(-300, std::min(300, ex)));
+    for (int c = 0; c < 4; ++c) {
+        so.v[c].assign((size_t)ns, c < 3 ? kFar : 0.0);
+        for (int64_t t = 0; t < ns; ++t) {
+            const int32_t i = so.perm[t];
+            if (i >= 0) so.v[c][t] = c < 3 ? pts[3 * (int64_t)i + c] * scale : w[i] * scale * scale;
+        }
+    }
+    for (size_t t = 0; t < so.tiles.size(); ++t)
+        for (int c = 0; c < 3; ++c) {
+            double a = INFINITY, b = -INFINITY;
+            for (int64_t e = (int64_t)t * kTB; e < (int64_t)(t + 1) * kTB && so.perm[e] >= 0; ++e) {
+                a = std::min(a, so.v[c][e]);
+                b = std::max(b, so.v[c][e]);
+            }
+            so.tiles[t].o[c] = a == b ? a : 0.5 * (a + b);  // exactly the plane's along its axis
+        }
+    return so;
+}
+
+}  // namespace
+
 bie_geom* geom_create(const double* pts, const double* nrm, const double* w, const double* diag, int64_t n,
                       int32_t npanels, int32_t nb, const int32_t* rowptr, const int32_t* col, const double* val,
                       int64_t nblocks, int device) {
@@ -1274,35 +1412,12 @@ bie_geom* geom_create(const double* pts, const double* nrm, const double* w, con
     }
     upload(g->w, w, n, s);
     upload(g->diag, diag, n, s);
-    // Morton (Z-order) permutation of the nodes: 21-bit quantised coordinates, bits interleaved
     {
-        double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-        for (int64_t i = 0; i < n; ++i)
-            for (int c = 0; c < 3; ++c) {
-                lo[c] = std::min(lo[c], pts[3 * i + c]);
-                hi[c] = std::max(hi[c], pts[3 * i + c]);
-            }
-        const double ext = std::max({hi[0] - lo[0], hi[1] - lo[1], hi[2] - lo[2], 1e-300});
-        auto spread = [](uint64_t v) {  // 21 bits -> every third bit of 63
-            v &= 0x1FFFFFull;
-            v = (v | v << 32) & 0x1F00000000FFFFull;
-            v = (v | v << 16) & 0x1F0000FF0000FFull;
-            v = (v | v << 8) & 0x100F00F00F00F00Full;
-            v = (v | v << 4) & 0x10C30C30C30C30C3ull;
-            v = (v | v << 2) & 0x1249249249249249ull;
-            return v;
-        };
-        std::vector<std::pair<uint64_t, int32_t>> key((size_t)n);
-        for (int64_t i = 0; i < n; ++i) {
-            uint64_t q[3];
-            for (int c = 0; c < 3; ++c)
-                q[c] = (uint64_t)std::min(2097151.0, std::floor((pts[3 * i + c] - lo[c]) / ext * 2097151.0));
-            key[i] = {spread(q[0]) | spread(q[1]) << 1 | spread(q[2]) << 2, (int32_t)i};
-        }
-        std::stable_sort(key.begin(), key.end(), [](auto& a, auto& b) { return a.first < b.first; });
-        std::vector<int32_t> perm((size_t)n);
-        for (int64_t i = 0; i < n; ++i) perm[i] = key[i].second;
-        upload(g->perm, perm.data(), n, s);
+        const SortedNodes so = sort_nodes(pts, nrm, w, n);
+        g->ns = (int64_t)so.perm.size();
+        for (int c = 0; c < 4; ++c) upload(c == 0 ? g->sx : (c == 1 ? g->sy : (c == 2 ? g->sz : g->sw)), so.v[c].data(), g->ns, s);
+        upload(g->perm, so.perm.data(), g->ns, s);
+        upload(g->tiles, so.tiles.data(), so.tiles.size(), s);
         BIE_CK(cudaStreamSynchronize(s));
     }
     g->errflag.ensure(sizeof(int));
@@ -1316,7 +1431,7 @@ bie_geom* geom_create(const double* pts, const double* nrm, const double* w, con
         upload(g->val, val, (size_t)nblocks * nb * nb, s);
     }
     BIE_CK(cudaStreamSynchronize(s));
-    g->geom_bytes = sizeof(double) * (size_t)n * 9 + (nblocks > 0 ? (sizeof(int32_t) * ((size_t)npanels + 1 + nblocks) +
+    g->geom_bytes = sizeof(double) * ((size_t)n * 8 + (size_t)g->ns * 4) + sizeof(int32_t) * (size_t)g->ns + (nblocks > 0 ? (sizeof(int32_t) * ((size_t)npanels + 1 + nblocks) +
                                                                      sizeof(double) * (size_t)nblocks * nb * nb)
                                                                   : 0);
     return g.release();
@@ -1398,7 +1513,8 @@ void geom_destroy(bie_geom* g) {
         DeviceGuard dg(g->device);
         if (g->stream) cudaStreamSynchronize(g->stream);
         if (g->s_ls) cudaStreamSynchronize(g->s_ls);
-        bie::Buf* all[] = {&g->x, &g->y, &g->z, &g->nx, &g->ny, &g->nz, &g->w, &g->diag, &g->pinv, &g->perm, &g->rowptr,
+        bie::Buf* all[] = {&g->x, &g->y, &g->z, &g->nx, &g->ny, &g->nz, &g->w, &g->diag, &g->pinv, &g->sx, &g->sy, &g->sz, &g->sw,
+                           &g->perm, &g->tiles, &g->rowptr,
                            &g->col, &g->val, &g->part, &g->small, &g->bpack, &g->errflag, &g->cpart, &g->V, &g->W, &g->R, &g->gv, &g->cs, &g->sn,
                            &g->h, &g->h2, &g->hn, &g->beta, &g->eps, &g->active, &g->jlast, &g->yv, &g->resid,
                            &g->dpart, &g->rr, &g->xo, &g->dd, &g->io_a, &g->io_b, &g->sol, &g->srcpack, &g->glist,
@@ -1859,10 +1975,10 @@ void group_apply_tc(const std::vector<Member*>& ms, const std::vector<const doub
         const int k = ms[i]->k;
         sp[i] = tc_split(g, k, pieces);
         g->part.ensure(sizeof(float) * (size_t)sp[i].nsplit * g->n * k);
-        g->bpack.ensure(block_tc_pack_bytes(g->n, k, pieces));
+        g->bpack.ensure(block_tc_pack_bytes(g->ns, k, pieces));
         tm.push_back(TcMember{gdev(g), X[i], k, 0, k, nullptr, sp[i].nsplit, sp[i].chunk, g->part.as<float>(), k,
                               g->bpack.as<uint8_t>()});
-        nitems += ((g->n + kTcTileM - 1) / kTcTileM) * sp[i].nsplit;
+        nitems += (g->ns / kTcTileM) * sp[i].nsplit;
     }
     bie_geom* lead = ms.front()->g;
     const size_t need = block_tc_list_bytes((int)ms.size(), nitems);
