@@ -109,18 +109,16 @@ __device__ __forceinline__ double over_r3(double r2) {
 // K3 (blocktc.cu): tensor-core block direct sum for columns [c0, c0 + kc), kc <= 128,
 // kernel and right-hand sides split into `pieces` bf16 pieces (2 or 3).
 void launch_block_tc(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,
-                     int64_t cps, float* part, int ldp, uint8_t* bpack, int* err, int pieces, int force_ctas,
-                     cudaStream_t s);
+                     float* part, int ldp, uint8_t* bpack, int* err, int pieces, cudaStream_t s);
 size_t block_tc_pack_bytes(int64_t slots, int kc, int pieces);
 // One geometry's share of a K3 work-list launch: columns [c0, c0 + kc) (kc <= 128) of X,
-// nsplit source splits of cps chunks, partials into part (ldp), Q images into bpack.
+// nsplit source splits, partials into part (ldp), Q images into bpack.
 struct TcMember {
     GeomDev g;
     const double* X;
     int ldx, c0, kc;
     const double* pre;
     int nsplit;
-    int64_t cps;
     float* part;
     int ldp;
     uint8_t* bpack;
@@ -131,7 +129,7 @@ struct TcMember {
 void launch_block_tc_list(const std::vector<TcMember>& ms, int pieces, int* err, void* dscratch, size_t scratch_bytes,
                           cudaStream_t s);
 size_t block_tc_list_bytes(int nmembers, int64_t nitems);
-int block_tc_ctas_per_sm(int kc, int pieces, int force_ctas = 0);
+int block_tc_ctas_per_sm(int kc, int pieces);
 int tc_npad(int kc);
 // K1 with the FP64 tensor-core contraction (dt64mma.cu), columns [c0, c0 + kc), kc <= 64.
 void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,

@@ -411,12 +411,11 @@ Split direct_sum(bie_geom* g, Kern kind, const double* X, int ldx, int k, const 
 // K3 launch plan: the number of source splits ns (<= 16, and at most 1024 chunks
 // per split) that minimises the time of the wave-quantised grid, which is
 // proportional to ceil(tiles ns / slots) / ns; ties go to fewer splits (each
-// split adds an FP32 partial for the combine to read). force_ctas selects the CTA
-// shape (0 = default).
-Split tc_split(const bie_geom* g, int kc, int pieces, int force_ctas = 0) {
+// split adds an FP32 partial for the combine to read).
+Split tc_split(const bie_geom* g, int kc, int pieces) {
     const int64_t tiles = g->ns / kTcTileM;
     const int64_t chunks = g->ns / kTcChunk;
-    const int64_t slots = (int64_t)g->sms * block_tc_ctas_per_sm(kc, pieces, force_ctas);
+    const int64_t slots = (int64_t)g->sms * block_tc_ctas_per_sm(kc, pieces);
     const int64_t ns_min = std::min<int64_t>(chunks, std::max<int64_t>(1, (chunks + 1023) / 1024));
     const int64_t ns_max = std::min<int64_t>(chunks, std::max<int64_t>(ns_min, 16));
     int64_t ns = ns_min;
@@ -448,45 +447,35 @@ Split direct_sum_tc(bie_geom* g, const double* X, int k, const double* pre, int 
     GeomDev gd = gdev(g);
     const int kc0 = std::min(k, 128);
     const double npairs = (double)g->n * (g->n - 1);
-    auto run = [&](const Split& sp, int ctas, bool prof) {
+    auto run = [&](const Split& sp, bool prof) {
         g->part.ensure(sizeof(float) * (size_t)sp.nsplit * g->n * k);
         g->bpack.ensure(block_tc_pack_bytes(g->ns, kc0, pieces));
         for (int c0 = 0; c0 < k; c0 += 128) {
             int kc = std::min(128, k - c0);
             std::unique_ptr<Prof> pf;
             if (prof) pf.reset(new Prof(g, BIE_KERNEL_DIRECT_TC, s, 2, npairs, npairs * tc_npad(kc)));
-            launch_block_tc(gd, X, k, c0, kc, pre, sp.nsplit, sp.chunk, g->part.as<float>(), k,
-                            g->bpack.as<uint8_t>(), g->errflag.as<int>(), pieces, ctas, s);
+            launch_block_tc(gd, X, k, c0, kc, pre, sp.nsplit, g->part.as<float>(), k, g->bpack.as<uint8_t>(),
+                            g->errflag.as<int>(), pieces, s);
         }
     };
     const auto key = tune_key(0, kc0, pieces);
     auto it = g->tuned.find(key);
     if (it == g->tuned.end() && can_tune(g, s)) {
         std::vector<bie_geom::Tuned> cands;
-        const int shape0 = block_tc_ctas_per_sm(kc0, pieces, 0);
-        for (int ctas : {shape0, shape0 == 2 ? 1 : 0}) {
-            if (ctas == 0) continue;
-            const Split base = tc_split(g, kc0, pieces, ctas);
-            for (int64_t ns : {(int64_t)base.nsplit, (int64_t)base.nsplit / 2, 2 * (int64_t)base.nsplit}) {
-                const Split sp = ns == base.nsplit ? base : tc_split_n(g, ns);
-                bool dup = false;
-                for (auto& c : cands) dup = dup || (c.nsplit == sp.nsplit && c.ctas == ctas);
-                if (!dup) cands.push_back({sp.nsplit, sp.chunk, ctas, 0.0});
-            }
+        const int ctas = block_tc_ctas_per_sm(kc0, pieces);
+        const Split base = tc_split(g, kc0, pieces);
+        for (int64_t ns : {(int64_t)base.nsplit, (int64_t)base.nsplit / 2, 2 * (int64_t)base.nsplit}) {
+            const Split sp = ns == base.nsplit ? base : tc_split_n(g, ns);
+            bool dup = false;
+            for (auto& c : cands) dup = dup || c.nsplit == sp.nsplit;
+            if (!dup) cands.push_back({sp.nsplit, sp.chunk, ctas, 0.0});
         }
         it = g->tuned.emplace(key, tune(g, s, cands, [&](const bie_geom::Tuned& c) {
-                                   run(Split{c.nsplit, c.chunk}, c.ctas, false);
+                                   run(Split{c.nsplit, c.chunk}, false);
                                })).first;
     }
-    Split sp;
-    int ctas = 0;
-    if (it != g->tuned.end()) {
-        sp = Split{it->second.nsplit, it->second.chunk};
-        ctas = it->second.ctas;
-    } else {
-        sp = tc_split(g, kc0, pieces);
-    }
-    run(sp, ctas, true);
+    const Split sp = it != g->tuned.end() ? Split{it->second.nsplit, it->second.chunk} : tc_split(g, kc0, pieces);
+    run(sp, true);
     return sp;
 }
 
@@ -1976,7 +1965,7 @@ void group_apply_tc(const std::vector<Member*>& ms, const std::vector<const doub
         sp[i] = tc_split(g, k, pieces);
         g->part.ensure(sizeof(float) * (size_t)sp[i].nsplit * g->n * k);
         g->bpack.ensure(block_tc_pack_bytes(g->ns, k, pieces));
-        tm.push_back(TcMember{gdev(g), X[i], k, 0, k, nullptr, sp[i].nsplit, sp[i].chunk, g->part.as<float>(), k,
+        tm.push_back(TcMember{gdev(g), X[i], k, 0, k, nullptr, sp[i].nsplit, g->part.as<float>(), k,
                               g->bpack.as<uint8_t>()});
         nitems += (g->ns / kTcTileM) * sp[i].nsplit;
     }
