@@ -11,6 +11,7 @@
 
 #include <algorithm>
 
+#include "arnoldi.cuh"
 #include "common.cuh"
 
 namespace bie {
@@ -695,37 +696,12 @@ __global__ void k_axpby(double a, const double* __restrict__ X, double b, double
     Y[e] = a * X[e] + b * Y[e];
 }
 
-// Givens step of iteration j for every active column (one thread per column).
-// R: [(m+1) x (m+1) x k] column j holds h[0..j+1]; cs/sn: [m x k]; gv: [(m+1) x k].
-__global__ void k_givens(double* __restrict__ R, const double* __restrict__ h /*[(j+1) x k]*/,
-                         const double* __restrict__ h2 /*[(j+1) x k], second Gram-Schmidt pass, or null*/,
-                         const double* __restrict__ hnorm /*[k]*/, double* __restrict__ cs, double* __restrict__ sn,
-                         double* __restrict__ gv, int* __restrict__ active, int* __restrict__ jlast,
-                         const double* __restrict__ eps, double* __restrict__ resid, int j, int m1, int k) {
-    int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= k) return;
-    if (!active[c]) return;
-    double* Rj = R + ((int64_t)j * m1) * k;  // column j: Rj[i * k + c]
-    for (int i = 0; i <= j; ++i) Rj[i * k + c] = h[i * k + c] + (h2 ? h2[i * k + c] : 0.0);
-    Rj[(j + 1) * k + c] = hnorm[c];
-    for (int i = 0; i < j; ++i) {
-        double a = Rj[i * k + c], b = Rj[(i + 1) * k + c];
-        double ci = cs[i * k + c], si = sn[i * k + c];
-        Rj[i * k + c] = ci * a + si * b;
-        Rj[(i + 1) * k + c] = -si * a + ci * b;
-    }
-    double a = Rj[j * k + c], b = Rj[(j + 1) * k + c];
-    double r = hypot(a, b);
-    double cj = r > 0 ? a / r : 1.0, sj = r > 0 ? b / r : 0.0;
-    cs[j * k + c] = cj; sn[j * k + c] = sj;
-    Rj[j * k + c] = r; Rj[(j + 1) * k + c] = 0.0;
-    double gj = gv[j * k + c];
-    gv[(j + 1) * k + c] = -sj * gj;
-    gv[j * k + c] = cj * gj;
-    double res = fabs(gv[(j + 1) * k + c]);
-    resid[c] = res;
-    jlast[c] = j + 1;
-    if (res <= eps[c] || hnorm[c] == 0.0) active[c] = 0;
+// Givens step of iteration j for every active column (one thread per column); h (and h2 from a second
+// Gram-Schmidt pass, or null): [(j+1) x k], hnorm: [k].
+__global__ void k_givens(Givens G, const double* __restrict__ h, const double* __restrict__ h2,
+                         const double* __restrict__ hnorm, int j) {
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c < G.k) givens_column(G, c, h + c, h2 ? h2 + c : nullptr, G.k, hnorm[c], j);
 }
 
 // y = R^{-1} g for each column over its own jlast[c] (one thread per column).

@@ -628,6 +628,40 @@ void col_norms(bie_geom* g, const double* X, int k, double* out, cudaStream_t s)
     dots(g, X, 0, 1, X, k, out, 2, s);
 }
 
+// Orthogonalisation step j of the per-column GMRES: W against V_0 .. V_j by classical Gram-Schmidt
+// (passes: 1 or 2; the last one fused with the norm of the new direction), V_{j+1} and the columns'
+// Givens update, where the second pass's coefficients are added to the first's.
+void arnoldi_step(bie_geom* g, double* V, double* W, int j, int k, int m1, int passes, cudaStream_t s) {
+    const int64_t n = g->n, nk = n * (int64_t)k;
+    const Givens G{g->R.as<double>(), g->cs.as<double>(), g->sn.as<double>(), g->gv.as<double>(), g->active.as<int>(),
+                   g->jlast.as<int>(), g->eps.as<double>(), g->resid.as<double>(), m1, k};
+    if (nk <= kArnElems && k <= kArnCols) {
+        const size_t sm = arn_smem(n, k, j + 1);
+        if (sm <= 200 * 1024) {
+            ensure_smem_limit((const void*)k_arnoldi_cluster, sm);
+            Prof pf(g, BIE_KERNEL_KRYLOV, s);
+            k_arnoldi_cluster<<<kArnCtas, kArnThreads, sm, s>>>(W, V, nk, j, n, passes, G);
+            BIE_CK(cudaGetLastError());
+            return;
+        }
+    }
+    double* h = g->h.as<double>();
+    double* h2 = passes > 1 ? g->h2.as<double>() : nullptr;
+    dots(g, V, nk, j + 1, W, k, h, 0, s);
+    if (h2) {
+        {
+            Prof pf(g, BIE_KERNEL_KRYLOV, s);
+            k_gs_update<<<grid1(nk), 256, 0, s>>>(W, V, nk, j + 1, h, n, k);
+        }
+        dots(g, V, nk, j + 1, W, k, h2, 0, s);
+    }
+    gs_update_norm(g, W, V, nk, j + 1, h2 ? h2 : h, k, g->hn.as<double>(), s);
+    Prof pf(g, BIE_KERNEL_KRYLOV, s, 2);
+    k_scale_cols<<<grid1(nk), 256, 0, s>>>(W, g->hn.as<double>(), n, k, V + (size_t)(j + 1) * nk);
+    k_givens<<<grid1(k, 64), 64, 0, s>>>(G, h, h2, g->hn.as<double>(), j);
+    BIE_CK(cudaGetLastError());
+}
+
 template <class T>
 void d2h(T* dst, const void* src, size_t count, cudaStream_t s) {
     BIE_CK(cudaMemcpyAsync(dst, src, sizeof(T) * count, cudaMemcpyDeviceToHost, s));
@@ -774,33 +808,7 @@ GmresResult gmres(bie_geom* g, const double* dr, double* dx, int k, int prec, ui
             auto iteration = [&]() {
                 double* Vj = V + (size_t)j * nk;
                 apply_op(g, Vj, W, k, prec, flags, pre, s);
-                // classical Gram-Schmidt, twice for FP64 solves; the last pass is fused with the
-                // norm of the new direction, and the second pass's coefficients are added to the
-                // first pass's in the Givens step
-                dots(g, V, nk, j + 1, W, k, g->h.as<double>(), 0, s);
-                if (one_pass) {
-                    gs_update_norm(g, W, V, nk, j + 1, g->h.as<double>(), k, g->hn.as<double>(), s);
-                } else {
-                    {
-                        Prof pf(g, BIE_KERNEL_KRYLOV, s);
-                        k_gs_update<<<grid1(nk), 256, 0, s>>>(W, V, nk, j + 1, g->h.as<double>(), n, k);
-                    }
-                    dots(g, V, nk, j + 1, W, k, g->h2.as<double>(), 0, s);
-                    gs_update_norm(g, W, V, nk, j + 1, g->h2.as<double>(), k, g->hn.as<double>(), s);
-                }
-                {
-                    Prof pf(g, BIE_KERNEL_KRYLOV, s);
-                    k_scale_cols<<<grid1(nk), 256, 0, s>>>(W, g->hn.as<double>(), n, k, V + (size_t)(j + 1) * nk);
-                }
-                {
-                    Prof pf(g, BIE_KERNEL_KRYLOV, s);
-                    k_givens<<<grid1(k, 64), 64, 0, s>>>(g->R.as<double>(), g->h.as<double>(),
-                                                        one_pass ? nullptr : g->h2.as<double>(),
-                                                        g->hn.as<double>(), g->cs.as<double>(), g->sn.as<double>(),
-                                                        g->gv.as<double>(), g->active.as<int>(), g->jlast.as<int>(),
-                                                        g->eps.as<double>(), g->resid.as<double>(), j, m1, k);
-                }
-                BIE_CK(cudaGetLastError());
+                arnoldi_step(g, V, W, j, k, m1, one_pass ? 1 : 2, s);
             };
             ++res.matvecs;
             if (use_graph && !gc->exec[j]) {
@@ -2100,17 +2108,7 @@ void group_gmres(const std::vector<Member*>& all, int pieces, uint32_t flags, in
             for (Member* M : run) {
                 bie_geom* g = M->g;
                 const int k = M->k;
-                const int64_t nk = g->n * (int64_t)k;
-                double* V = g->V.as<double>();
-                double* W = g->W.as<double>();
-                dots(g, V, nk, j + 1, W, k, g->h.as<double>(), 0, s);
-                gs_update_norm(g, W, V, nk, j + 1, g->h.as<double>(), k, g->hn.as<double>(), s);
-                k_scale_cols<<<grid1(nk), 256, 0, s>>>(W, g->hn.as<double>(), g->n, k, V + (size_t)(j + 1) * nk);
-                k_givens<<<grid1(k, 64), 64, 0, s>>>(g->R.as<double>(), g->h.as<double>(), nullptr, g->hn.as<double>(),
-                                                    g->cs.as<double>(), g->sn.as<double>(), g->gv.as<double>(),
-                                                    g->active.as<int>(), g->jlast.as<int>(), g->eps.as<double>(),
-                                                    g->resid.as<double>(), j, m1, k);
-                BIE_CK(cudaGetLastError());
+                arnoldi_step(g, g->V.as<double>(), g->W.as<double>(), j, k, m1, 1, s);
                 M->lpmv += 1;
                 M->it += 1;
             }
