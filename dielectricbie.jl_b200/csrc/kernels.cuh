@@ -333,7 +333,7 @@ __global__ void k_combine(int64_t n, int k, const TP* __restrict__ part, int nsp
 // loads feeds R FMAs, and the R block values are warp-wide broadcasts. Then
 //   Y[i][c] = (1/4pi) sum_s part[s][i][c] + sum_b B . (p X) + t_i p_i X[i][c].
 // ---------------------------------------------------------------------------
-// K4 (block-row form): one CTA per (target panel P, 32-column tile). The BSR
+// K4 (block-row form): one CTA of CT / 8 warps per (target panel P, CT-column tile). The BSR
 // blocks of the panel's row, C_b (nb x nb, column-major), multiply the slabs
 // p .* X[source panel of b] on the FP64 tensor path (mma.sync m8n8k4 f64; a
 // warp owns one 8-column n-tile and the panel's MT 8-row m-tiles); blocks and
@@ -362,7 +362,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-constexpr int kCombTile = 32;  // columns per CTA
 
 // Slab row stride for a kt-column tile: kt rounded up to 8, plus 4 (stride = 4 or 12
 // mod 16 doubles, so a half-warp's fragment loads hit distinct banks).
@@ -370,29 +369,32 @@ __host__ __device__ inline int comb_ldx(int kt) { return ((kt + 7) / 8) * 8 + 4;
 
 // Shared memory of the block-row combine for nb-row panels, kt-column tiles and
 // `stages` pipeline stages (reused for the warps' final reduction).
-inline size_t combine_smem_bytes(int nb, int kt, int stages) {
+inline size_t combine_smem_bytes(int nb, int kt, int stages, int warps) {
     const int mt = (nb + 7) / 8, kp = ((nb + 3) / 4) * 4;
     const int ldc = mt * 8 + 4;
     const size_t pipe = (size_t)stages * kp * (ldc + comb_ldx(kt) + 1);
-    const size_t red = (size_t)4 * mt * 2 * 32;  // cross-warp reduction of the accumulators
+    const size_t red = (size_t)warps * mt * 2 * 32;  // cross-warp reduction of the accumulators
     return sizeof(double) * std::max(pipe, red);
 }
 
 // With gsum != nullptr the panel's block list is split into groups of bpg blocks
 // (blockIdx.z = group) and each group writes its block sum to gsum[z][i][c]; the
 // reduction over groups, split partials and diagonal is then k_combine_groups.
-template <int MT, int NST, typename TP>
-__global__ void __launch_bounds__(128) k_combine_dmma(int64_t n, int k, const TP* __restrict__ part, int nsplit,
+// NB: nb at compile time (0: read at run time), so that the copies' index divisions are by constants; with a
+// full column tile the slab's are too.
+template <int MT, int NST, int NB, int CT, typename TP>
+__global__ void __launch_bounds__(4 * CT) k_combine_dmma(int64_t n, int k, const TP* __restrict__ part, int nsplit,
                                                       const double* __restrict__ X, const double* __restrict__ pre,
                                                       const double* __restrict__ diag,
                                                       const int32_t* __restrict__ rowptr,
                                                       const int32_t* __restrict__ col,
-                                                      const double* __restrict__ val, int nb,
+                                                      const double* __restrict__ val, int nb_,
                                                       double* __restrict__ Y, int bpg, double* __restrict__ gsum) {
+    const int nb = NB ? NB : nb_;
     // column stride of a staged block: MT * 8 rows + 4 (= 4 or 12 mod 16 doubles)
     constexpr int LDC = MT * 8 + 4;
-    const int c0 = blockIdx.y * kCombTile;
-    const int kt = min(kCombTile, k - c0);
+    const int c0 = blockIdx.y * CT;
+    const int kt = min(CT, k - c0);
     const int LDX = comb_ldx(kt);
     const int KS = (nb + 3) / 4, KP = KS * 4;
     const int SSTR = KP * (LDC + LDX + 1);  // doubles per pipeline stage
@@ -432,7 +434,13 @@ __global__ void __launch_bounds__(128) k_combine_dmma(int64_t n, int k, const TP
         }
         const int64_t base = (int64_t)col[b] * nb;
         double* dX = dC + KP * LDC;
-        if (x16) {
+        if (x16 && kt == CT) {
+            constexpr int h = CT / 2;
+            for (int e = threadIdx.x; e < nb * h; e += blockDim.x) {
+                const int q = e / h, cc = (e - q * h) * 2;
+                cp_async16(dX + q * LDX + cc, X + (base + q) * k + c0 + cc);
+            }
+        } else if (x16) {
             const int h = kt >> 1;
             for (int e = threadIdx.x; e < nb * h; e += blockDim.x) {
                 const int q = e / h, cc = (e - q * h) * 2;
@@ -452,8 +460,8 @@ __global__ void __launch_bounds__(128) k_combine_dmma(int64_t n, int k, const TP
     // n-tile split the block's k-steps (each keeps all MT accumulator chains busy) and
     // their partial sums are added through shared memory at the end
     const int ntiles = (kt + 7) / 8;
-    const int nw = ntiles >= 4 ? 4 : ntiles;  // distinct n-tiles in use
-    const int ksplit = 4 / nw;                // 1, 2 or 4 (nw = 3: one warp idle)
+    const int nw = ntiles >= CT / 8 ? CT / 8 : ntiles;  // distinct n-tiles in use
+    const int ksplit = (CT / 8) / nw;                   // leftover warps idle
     const int nt = warp % nw, kq = warp / nw;
     const bool wact = kq < ksplit;
     double acc[MT][2];

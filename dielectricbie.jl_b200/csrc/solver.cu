@@ -489,10 +489,23 @@ void combine(bie_geom* g, const TP* part, int nsplit, const double* X, double* Y
     const double* vl = corr ? g->val.as<double>() : nullptr;
     const int mt = (g->nb + 7) / 8;
     const bool panel_rows = g->nb > 0 && (int64_t)g->npanels * g->nb == g->n;
+    // Loads straight into fragments for 16-node panels and, at 36 nodes, for up to 16 columns on few
+    // panels (more are HBM-bound: streaming form below) and for 17 to 24 columns on many (us a launch
+    // with the events around it, before and after: 160 panels of 16, 1 column 20.2 and 12.6, 64 columns
+    // 45.5 and 29.0; 640 panels of 36, 8 columns 31.1 and 22.6, but 1,168 panels 38.7 and 43.5; 19
+    // columns, 1,168 panels 70.6 and 58.8, but 96 panels 21.7 and 22.9)
+    const bool direct = g->nb == 16 || (g->nb == 36 && (k <= 16 ? g->npanels < 6 * g->sms : k <= 24 && g->npanels >= 4 * g->sms));
+    if (panel_rows && direct && !std::getenv("BIE_COMBINE_ROWS") &&
+        launch_combine_direct<TP>(g->n, k, g->nb, g->npanels, part, nsplit, X, pre, dgp, rp, cl, vl, Y, s))
+        return;
     if (panel_rows && mt <= 8) {
         // the block products on the FP64 tensor path, two pipeline stages
-        const int nst = 2;
-        const size_t sm = combine_smem_bytes(g->nb, std::min(k, kCombTile), nst);
+        
+        // 64 columns a CTA read the blocks once instead of twice, at three CTAs per SM instead of four:
+        // 128 columns, 1,168 panels of 36: 197 us instead of 223; 64 columns: 126 instead of 121 there,
+        // 272 instead of 331 on 2,632 panels
+        const int ct = k > 64 || (k == 64 && g->npanels >= 12 * g->sms) ? 64 : 32;
+        const size_t sm = combine_smem_bytes(g->nb, std::min(k, ct), 2, ct / 8);
         // narrow blocks of right-hand sides on meshes with enough block rows to fill the
         // GPU: the HBM-bound streaming form, where its layout conditions hold
         // (BIE_COMBINE_ROWS forces the block-row form, for comparisons)
@@ -502,7 +515,7 @@ void combine(bie_geom* g, const TP* part, int nsplit, const double* X, double* Y
             BIE_CK(cudaGetLastError());
             return;
         }
-        const int64_t ctas = (int64_t)g->npanels * ((k + kCombTile - 1) / kCombTile);
+        const int64_t ctas = (int64_t)g->npanels * ((k + ct - 1) / ct);
         // long block rows of few panels: split each row into groups of blocks so that
         // about 8 CTAs per SM run (summed by k_combine_groups)
         int ngroups = 1, bpg = 0;
@@ -518,25 +531,35 @@ void combine(bie_geom* g, const TP* part, int nsplit, const double* X, double* Y
             g->cpart.ensure(sizeof(double) * (size_t)ngroups * g->n * k);
             gsum = g->cpart.as<double>();
         }
-        dim3 grid((unsigned)g->npanels, (unsigned)((k + kCombTile - 1) / kCombTile), (unsigned)ngroups);
-#define BIE_COMB(MT, NST)                                       \
-    ensure_smem_limit((const void*)k_combine_dmma<MT, NST, TP>, sm); \
-    k_combine_dmma<MT, NST, TP><<<grid, 128, sm, s>>>(g->n, k, part, nsplit, X, pre, dgp, rp, cl, vl, g->nb, Y, bpg, \
-                                                      gsum)
-#define BIE_COMB_MT(NST)                      \
-    switch (mt) {                             \
-        case 1: BIE_COMB(1, NST); break;      \
-        case 2: BIE_COMB(2, NST); break;      \
-        case 3: BIE_COMB(3, NST); break;      \
-        case 4: BIE_COMB(4, NST); break;      \
-        case 5: BIE_COMB(5, NST); break;      \
-        case 6: BIE_COMB(6, NST); break;      \
-        case 7: BIE_COMB(7, NST); break;      \
-        default: BIE_COMB(8, NST); break;     \
+        dim3 grid((unsigned)g->npanels, (unsigned)((k + ct - 1) / ct), (unsigned)ngroups);
+#define BIE_COMB_CT(MT, NB, CT)                                        \
+    ensure_smem_limit((const void*)k_combine_dmma<MT, 2, NB, CT, TP>, sm); \
+    k_combine_dmma<MT, 2, NB, CT, TP><<<grid, 4 * CT, sm, s>>>(g->n, k, part, nsplit, X, pre, dgp, rp, cl, vl, g->nb, Y, \
+                                                               bpg, gsum)
+#define BIE_COMB(MT, NB)               \
+    if (ct == 64) {                    \
+        BIE_COMB_CT(MT, NB, 64);       \
+    } else {                           \
+        BIE_COMB_CT(MT, NB, 32);       \
     }
-        BIE_COMB_MT(2)
-#undef BIE_COMB_MT
+        switch (mt) {
+            case 1: BIE_COMB(1, 0); break;
+            case 2: BIE_COMB(2, 0); break;
+            case 3: BIE_COMB(3, 0); break;
+            case 4: BIE_COMB(4, 0); break;
+            case 5:
+                if (g->nb == 36) {
+                    BIE_COMB(5, 36);
+                } else {
+                    BIE_COMB(5, 0);
+                }
+                break;
+            case 6: BIE_COMB(6, 0); break;
+            case 7: BIE_COMB(7, 0); break;
+            default: BIE_COMB(8, 0); break;
+        }
 #undef BIE_COMB
+#undef BIE_COMB_CT
         if (gsum) {
             BIE_CK(cudaGetLastError());
             const int64_t tot = g->n * (int64_t)k;

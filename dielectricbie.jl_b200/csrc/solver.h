@@ -61,6 +61,12 @@ template <typename TP>
 bool launch_combine_bulk(int64_t n, int k, int nb, int npanels, const TP* part, int nsplit, const double* X,
                          const double* pre, const double* diag, const int32_t* rowptr, const int32_t* col,
                          const double* val, double* Y, int* err, int sms, cudaStream_t s);
+// K4 for panels of 16 nodes, or 36 with up to 24 columns (combine_direct.cu); returns false (nothing
+// launched) for others.
+template <typename TP>
+bool launch_combine_direct(int64_t n, int k, int nb, int npanels, const TP* part, int nsplit, const double* X,
+                           const double* pre, const double* diag, const int32_t* rowptr, const int32_t* col,
+                           const double* val, double* Y, cudaStream_t s);
 // Near-accurate probe potentials on a device (probe.cu).
 struct ProbeSetup;
 struct ProbeDev;
