@@ -62,9 +62,12 @@ __device__ __forceinline__ void copy_commit() { asm volatile("cp.async.commit_gr
 template <int N>
 __device__ __forceinline__ void copy_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// Kernel values: the adjoint double layer in a planar or another tile, the single layer 1 / r.
+enum Value { kPlanar, kGeneral, kSingle };
+
 // One source tile into the warp's accumulators. stg: the stage; cnt: its live sources; self:
 // the tile's first slot when it may hold one of the warp's own targets, else negative.
-template <int NC, bool PLANAR>
+template <int NC, Value V>
 __device__ __forceinline__ void tile_step(const double* __restrict__ stg, int cnt, double plane,
                                           const double (&ta)[mtw<NC>()], const double (&tb)[mtw<NC>()],
                                           const double (&tc)[mtw<NC>()], const double (&tn)[mtw<NC>()][3],
@@ -80,7 +83,7 @@ __device__ __forceinline__ void tile_step(const double* __restrict__ stg, int cn
         double wj = stg[3 * TSRC + j];
         if (has_pre) wj *= stg[4 * TSRC + j];
         double a[MTW];
-        if (PLANAR) {
+        if (V == kPlanar) {
             const double da = plane - sa, da2 = da * da;
             wj *= da;
 #pragma unroll
@@ -92,8 +95,11 @@ __device__ __forceinline__ void tile_step(const double* __restrict__ stg, int cn
 #pragma unroll
             for (int mt = 0; mt < MTW; ++mt) {
                 const double dx = ta[mt] - sa, dy = tb[mt] - sb, dz = tc[mt] - sc;
-                const double dn = fma(tn[mt][0], dx, fma(tn[mt][1], dy, tn[mt][2] * dz));
-                a[mt] = over_r3(fma(dx, dx, fma(dy, dy, dz * dz))) * (dn * wj);
+                const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                if (V == kSingle)
+                    a[mt] = rsqrt(r2) * wj;
+                else
+                    a[mt] = over_r3(r2) * (fma(tn[mt][0], dx, fma(tn[mt][1], dy, tn[mt][2] * dz)) * wj);
                 if (j >= cnt || (self >= 0 && self + j == slot0 + mt * 8)) a[mt] = 0.0;
             }
         }
@@ -107,16 +113,18 @@ __device__ __forceinline__ void tile_step(const double* __restrict__ stg, int cn
     }
 }
 
-template <int NC>
-__global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const double* __restrict__ X, int ldx,
-                                                               int c0, int kc, const double* __restrict__ pre,
-                                                               double* __restrict__ part, int ldp) {
+// The sum's body. POT: the single-layer potential at M targets T (3 x M) instead of the adjoint double
+// layer at the nodes.
+template <int NC, bool POT>
+__device__ __forceinline__ void sum_body(const GeomDev& g, const double* __restrict__ T, int64_t M,
+                                         const double* __restrict__ X, int ldx, int c0, int kc,
+                                         const double* __restrict__ pre, double* __restrict__ part, int ldp) {
     constexpr int MTW = mtw<NC>(), LDQ = ldq<NC>(), TB = 32 * MTW;
     extern __shared__ __align__(16) double ring[];  // [NST][stage_doubles]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = lane >> 2, kq = lane & 3;
     const int64_t t0 = (int64_t)blockIdx.x * TB;
-    const TileInfo ti = g.tiles ? g.tiles[t0 / kTB] : TileInfo{3, 0, 0, {0.0, 0.0, 0.0}};
+    const TileInfo ti = !POT && g.tiles ? g.tiles[t0 / kTB] : TileInfo{3, 0, 0, {0.0, 0.0, 0.0}};
     // coordinate arrays, the tile's axis first
     const double* pa = ti.axis == 1 ? g.sy : (ti.axis == 2 ? g.sz : g.sx);
     const double* pb = ti.axis == 1 ? g.sz : (ti.axis == 2 ? g.sx : g.sy);
@@ -127,15 +135,21 @@ __global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const
 #pragma unroll
     for (int mt = 0; mt < MTW; ++mt) {
         const int64_t slot = slot0 + 8 * mt;
-        const int64_t i = slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1;
         ta[mt] = tb[mt] = tc[mt] = -kFar;  // no target: not stored
         tn[mt][0] = tn[mt][1] = tn[mt][2] = 0.0;
+        if (POT) {
+            if (slot < M) {
+                ta[mt] = T[3 * slot]; tb[mt] = T[3 * slot + 1]; tc[mt] = T[3 * slot + 2];
+            }
+            continue;
+        }
+        const int64_t i = slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1;
         if (i >= 0) {
             ta[mt] = pa[slot]; tb[mt] = pb[slot]; tc[mt] = pc[slot];
             tn[mt][0] = g.nx[i]; tn[mt][1] = g.ny[i]; tn[mt][2] = g.nz[i];
         }
     }
-    const double plane = pa[t0];
+    const double plane = POT ? 0.0 : pa[t0];
     double acc[MTW][NC / 8][2];
 #pragma unroll
     for (int mt = 0; mt < MTW; ++mt)
@@ -195,22 +209,25 @@ __global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const
         next = row_node(t + NST);
         const double* stg = ring + (t % NST) * stage_doubles<NC>();
         const int cnt = (int)min((int64_t)TSRC, l1 - l0 - (int64_t)t * TSRC);
-        if (ti.axis < 3) {
-            tile_step<NC, true>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, pre != nullptr, -1, slot0);
+        if (POT) {
+            tile_step<NC, kSingle>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, false, -1, slot0);
+        } else if (ti.axis < 3) {
+            tile_step<NC, kPlanar>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, pre != nullptr, -1, slot0);
         } else {
             const int64_t jt = live_slot(ti, l0 + (int64_t)t * TSRC);
             const bool self = jt < t0 + TB && jt + TSRC > t0;
-            tile_step<NC, false>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, pre != nullptr, self ? jt : -1, slot0);
+            tile_step<NC, kGeneral>(stg, cnt, plane, ta, tb, tc, tn, acc, lane, pre != nullptr, self ? jt : -1, slot0);
         }
     }
     // D fragment: (row grp, columns 2 kq, 2 kq + 1) of each (m-tile, n-tile)
 #pragma unroll
     for (int mt = 0; mt < MTW; ++mt) {
         const int64_t slot = slot0 + 8 * mt;
-        const int64_t i = slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1;
+        const int64_t i = POT ? (slot < M ? slot : -1)
+                              : (slot < g.ns ? (g.perm ? (int64_t)g.perm[slot] : slot) : -1);
         if (i < 0) continue;
         const double sgn = ti.axis == 0 ? g.nx[i] : (ti.axis == 1 ? g.ny[i] : (ti.axis == 2 ? g.nz[i] : 1.0));
-        double* o = part + ((int64_t)blockIdx.y * g.n + i) * ldp + c0;
+        double* o = part + ((int64_t)blockIdx.y * (POT ? M : g.n) + i) * ldp + c0;
 #pragma unroll
         for (int nt = 0; nt < NC / 8; ++nt) {
             const int c = nt * 8 + 2 * kq;
@@ -221,13 +238,37 @@ __global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const
 }
 
 template <int NC>
+__global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const double* __restrict__ X, int ldx,
+                                                               int c0, int kc, const double* __restrict__ pre,
+                                                               double* __restrict__ part, int ldp) {
+    sum_body<NC, false>(g, nullptr, 0, X, ldx, c0, kc, pre, part, ldp);
+}
+
+template <int NC>
+__global__ void __launch_bounds__(NTHR, occ<NC>()) k_pot_f64_mma(GeomDev g, const double* __restrict__ T, int64_t M,
+                                                                const double* __restrict__ X, int ldx, int c0, int kc,
+                                                                double* __restrict__ part, int ldp) {
+    sum_body<NC, true>(g, T, M, X, ldx, c0, kc, nullptr, part, ldp);
+}
+
+template <int NC> constexpr size_t smem() { return sizeof(double) * NST * stage_doubles<NC>(); }
+
+template <int NC>
 void launch(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit, double* part,
             int ldp, cudaStream_t s) {
     constexpr int TB = 32 * mtw<NC>();
-    const size_t sm = sizeof(double) * NST * stage_doubles<NC>();
-    ensure_smem_limit((const void*)k_dt_f64_mma<NC>, sm);
+    ensure_smem_limit((const void*)k_dt_f64_mma<NC>, smem<NC>());
     const dim3 grid((unsigned)((g.ns + TB - 1) / TB), (unsigned)nsplit);
-    k_dt_f64_mma<NC><<<grid, NTHR, sm, s>>>(g, X, ldx, c0, kc, pre, part, ldp);
+    k_dt_f64_mma<NC><<<grid, NTHR, smem<NC>(), s>>>(g, X, ldx, c0, kc, pre, part, ldp);
+}
+
+template <int NC>
+void launch_pot(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc, int nsplit,
+                double* part, int ldp, cudaStream_t s) {
+    constexpr int TB = 32 * mtw<NC>();
+    ensure_smem_limit((const void*)k_pot_f64_mma<NC>, smem<NC>());
+    const dim3 grid((unsigned)((M + TB - 1) / TB), (unsigned)nsplit);
+    k_pot_f64_mma<NC><<<grid, NTHR, smem<NC>(), s>>>(g, T, M, X, ldx, c0, kc, part, ldp);
 }
 
 }  // namespace d64
@@ -244,6 +285,37 @@ void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int k
         d64::launch<16>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
     else
         d64::launch<8>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
+    BIE_CK(cudaGetLastError());
+}
+
+// Source splits of the potential at M targets: the largest number that one wave of CTAs holds.
+int pot_f64_mma_splits(int64_t n, int64_t M, int k, int sms) {
+    const int kc = std::min(k, 64);
+    const int tb = 32 * (kc <= 16 ? d64::mtw<16>() : d64::mtw<64>()), per_sm = kc <= 32 ? d64::occ<32>() : d64::occ<64>();
+    const int64_t tiles = (M + tb - 1) / tb;
+    return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm / tiles, (n + kTS - 1) / kTS));
+}
+
+// Single-layer potential partials (laplace3d_pottrg, src/kernel/laplace3d.jl:69-82, without the
+// 1/(4 pi)) of columns [c0, c0 + kc), kc <= 64 and c0 a multiple of 64, at M targets T (3 x M):
+//   part[s][m][c0 + c] = sum_{j in split s} w_j X[j][c0 + c] / |x_m - y_j|
+// The same kernel with 1 / r for its value: 42,048 nodes, 1,000 targets, 64 columns 0.55 -> 0.27 ms with the split reduction, where
+// the sum on FP64 FMAs alone is limited by its shared-memory loads.
+void launch_pot_f64_mma(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc,
+                        int nsplit, double* part, int ldp, cudaStream_t s) {
+    GeomDev r = g;  // the nodes in the caller's order and unit: the targets are not scaled
+    r.sx = g.x; r.sy = g.y; r.sz = g.z; r.sw = g.w;
+    r.perm = nullptr;
+    r.tiles = nullptr;
+    r.ns = g.n;
+    if (kc > 32)
+        d64::launch_pot<64>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
+    else if (kc > 16)
+        d64::launch_pot<32>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
+    else if (kc > 8)
+        d64::launch_pot<16>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
+    else
+        d64::launch_pot<8>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
     BIE_CK(cudaGetLastError());
 }
 

@@ -192,15 +192,16 @@ void upload(bie::Buf& b, const T* src, size_t count, cudaStream_t s) {
 // --------------------------- direct-sum launchers --------------------------
 enum class Kern { DT64, DT32, POT64 };
 
-// Instances: DT64 with fewer than 8 columns (wider sums run dt64mma.cu's kernel), the others with
-// a power of two.
+// Instances: DT64 with fewer than 8 columns and POT64 with 1, 2 or 4 (wider sums run dt64mma.cu's
+// kernels), DT32 with a power of two.
 template <int C>
 void* kern_ptr(Kern kind) {
     if constexpr (C < 8)
         if (kind == Kern::DT64) return (void*)k_dt_f64<C>;
     if constexpr ((C & (C - 1)) == 0) {
         if (kind == Kern::DT32) return (void*)k_dt_f32<C>;
-        if (kind == Kern::POT64) return (void*)k_pot_f64<C>;
+        if constexpr (C < 8)
+            if (kind == Kern::POT64) return (void*)k_pot_f64<C>;
     }
     throw Error(BIE_EUNSUPPORTED, "no direct-sum kernel of this width");
 }
@@ -243,7 +244,8 @@ void launch_direct(Kern kind, const GeomDev& g, const double* X, int ldx, int c0
         if (kind == Kern::DT64) k_dt_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, pre, part, ldp);
     if constexpr ((C & (C - 1)) == 0) {
         if (kind == Kern::DT32) k_dt_f32<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, pre, part, ldp);
-        if (kind == Kern::POT64) k_pot_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, T, M, sp.chunk, part, ldp);
+        if constexpr (C < 8)
+            if (kind == Kern::POT64) k_pot_f64<C><<<grid, kTB, sm, s>>>(g, X, ldx, c0, T, M, sp.chunk, part, ldp);
     }
     BIE_CK(cudaGetLastError());
 }
@@ -377,6 +379,16 @@ Split direct_sum(bie_geom* g, Kern kind, const double* X, int ldx, int k, const 
         }
         const Split sp = it != g->tuned.end() ? Split{it->second.nsplit, it->second.chunk} : base;
         run(sp, true);
+        return sp;
+    }
+    if (kind == Kern::POT64 && k >= 8) {
+        const Split sp{pot_f64_mma_splits(g->n, M, k, g->sms), 0};
+        g->part.ensure(sizeof(double) * (size_t)sp.nsplit * M * k);
+        for (int c0 = 0; c0 < k; c0 += 64) {
+            const int kc = std::min(64, k - c0);
+            Prof pf(g, BIE_KERNEL_OTHER, s, 1, (double)M * g->n, (double)M * g->n * kc);
+            launch_pot_f64_mma(gd, T, M, X, ldx, c0, kc, sp.nsplit, g->part.as<double>(), k, s);
+        }
         return sp;
     }
     int64_t rows = kind == Kern::POT64 ? M : g->ns;
