@@ -33,9 +33,11 @@ constexpr int NTHR = 128;  // threads per CTA
 constexpr int TSRC = 32;   // sources per shared-memory tile
 constexpr int NST = 3;     // stages of the source ring
 
-// m-tiles per warp and resident CTAs per SM: the accumulators take MTW * NC / 4 doubles a thread
+// m-tiles per warp and resident CTAs per SM: the accumulators take MTW * NC / 4 doubles a thread. Four
+// m-tiles share the source's part of a value (8 columns, 42,048 nodes: 2.02 ms, two m-tiles 2.22); the
+// 8-column instance needs more than 128 registers to overlap its chains (three CTAs 2.02 ms, four 2.08).
 template <int NC> constexpr int mtw() { return NC <= 16 ? 4 : 2; }
-template <int NC> constexpr int occ() { return NC <= 32 ? 4 : 3; }
+template <int NC> constexpr int occ() { return NC > 8 && NC <= 32 ? 4 : 3; }
 // Row stride of a staged X tile (= 4 or 12 mod 16 doubles): the four k-rows a half-warp's
 // B-fragment load touches fall on distinct banks; rows stay 16-byte aligned.
 template <int NC> constexpr int ldq() { return NC + 4; }
@@ -113,12 +115,13 @@ __device__ __forceinline__ void tile_step(const double* __restrict__ stg, int cn
     }
 }
 
-// The sum's body. POT: the single-layer potential at M targets T (3 x M) instead of the adjoint double
+// POT: the single-layer potential at M targets T (3 x M) instead of the adjoint double
 // layer at the nodes.
 template <int NC, bool POT>
-__device__ __forceinline__ void sum_body(const GeomDev& g, const double* __restrict__ T, int64_t M,
-                                         const double* __restrict__ X, int ldx, int c0, int kc,
-                                         const double* __restrict__ pre, double* __restrict__ part, int ldp) {
+__global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const double* __restrict__ T, int64_t M,
+                                                               const double* __restrict__ X, int ldx, int c0, int kc,
+                                                               const double* __restrict__ pre,
+                                                               double* __restrict__ part, int ldp) {
     constexpr int MTW = mtw<NC>(), LDQ = ldq<NC>(), TB = 32 * MTW;
     extern __shared__ __align__(16) double ring[];  // [NST][stage_doubles]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -237,38 +240,30 @@ __device__ __forceinline__ void sum_body(const GeomDev& g, const double* __restr
     }
 }
 
-template <int NC>
-__global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const double* __restrict__ X, int ldx,
-                                                               int c0, int kc, const double* __restrict__ pre,
-                                                               double* __restrict__ part, int ldp) {
-    sum_body<NC, false>(g, nullptr, 0, X, ldx, c0, kc, pre, part, ldp);
-}
-
-template <int NC>
-__global__ void __launch_bounds__(NTHR, occ<NC>()) k_pot_f64_mma(GeomDev g, const double* __restrict__ T, int64_t M,
-                                                                const double* __restrict__ X, int ldx, int c0, int kc,
-                                                                double* __restrict__ part, int ldp) {
-    sum_body<NC, true>(g, T, M, X, ldx, c0, kc, nullptr, part, ldp);
-}
-
 template <int NC> constexpr size_t smem() { return sizeof(double) * NST * stage_doubles<NC>(); }
 
-template <int NC>
-void launch(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit, double* part,
-            int ldp, cudaStream_t s) {
+template <int NC, bool POT>
+void launch(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc, const double* pre,
+            int nsplit, double* part, int ldp, cudaStream_t s) {
     constexpr int TB = 32 * mtw<NC>();
-    ensure_smem_limit((const void*)k_dt_f64_mma<NC>, smem<NC>());
-    const dim3 grid((unsigned)((g.ns + TB - 1) / TB), (unsigned)nsplit);
-    k_dt_f64_mma<NC><<<grid, NTHR, smem<NC>(), s>>>(g, X, ldx, c0, kc, pre, part, ldp);
+    const auto k = k_dt_f64_mma<NC, POT>;
+    ensure_smem_limit((const void*)k, smem<NC>());
+    const dim3 grid((unsigned)(((POT ? M : g.ns) + TB - 1) / TB), (unsigned)nsplit);
+    k<<<grid, NTHR, smem<NC>(), s>>>(g, T, M, X, ldx, c0, kc, pre, part, ldp);
 }
 
-template <int NC>
-void launch_pot(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc, int nsplit,
-                double* part, int ldp, cudaStream_t s) {
-    constexpr int TB = 32 * mtw<NC>();
-    ensure_smem_limit((const void*)k_pot_f64_mma<NC>, smem<NC>());
-    const dim3 grid((unsigned)((M + TB - 1) / TB), (unsigned)nsplit);
-    k_pot_f64_mma<NC><<<grid, NTHR, smem<NC>(), s>>>(g, T, M, X, ldx, c0, kc, part, ldp);
+template <bool POT>
+void launch_width(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc,
+                  const double* pre, int nsplit, double* part, int ldp, cudaStream_t s) {
+    if (kc > 32)
+        launch<64, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
+    else if (kc > 16)
+        launch<32, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
+    else if (kc > 8)
+        launch<16, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
+    else
+        launch<8, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
+    BIE_CK(cudaGetLastError());
 }
 
 }  // namespace d64
@@ -277,15 +272,7 @@ void launch_pot(const GeomDev& g, const double* T, int64_t M, const double* X, i
 // of 64. The sources are split evenly into nsplit parts, each writing its own partial.
 void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,
                        double* part, int ldp, cudaStream_t s) {
-    if (kc > 32)
-        d64::launch<64>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    else if (kc > 16)
-        d64::launch<32>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    else if (kc > 8)
-        d64::launch<16>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    else
-        d64::launch<8>(g, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    BIE_CK(cudaGetLastError());
+    d64::launch_width<false>(g, nullptr, 0, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
 }
 
 // Source splits of the potential at M targets: the largest number that one wave of CTAs holds.
@@ -308,15 +295,7 @@ void launch_pot_f64_mma(const GeomDev& g, const double* T, int64_t M, const doub
     r.perm = nullptr;
     r.tiles = nullptr;
     r.ns = g.n;
-    if (kc > 32)
-        d64::launch_pot<64>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
-    else if (kc > 16)
-        d64::launch_pot<32>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
-    else if (kc > 8)
-        d64::launch_pot<16>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
-    else
-        d64::launch_pot<8>(r, T, M, X, ldx, c0, kc, nsplit, part, ldp, s);
-    BIE_CK(cudaGetLastError());
+    d64::launch_width<true>(r, T, M, X, ldx, c0, kc, nullptr, nsplit, part, ldp, s);
 }
 
 }  // namespace bie
