@@ -9,6 +9,7 @@
 #include <tuple>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -1290,6 +1291,8 @@ void check_prec(int prec) {
 // ---------------------------------------------------------------------------
 namespace {
 
+std::atomic<int64_t> g_geoms{0};  // geometries alive
+
 // The sorted order of the direct sums (GeomDev): scaled positions and weights, the node of each
 // slot, and each tile's plane and origin.
 struct SortedNodes {
@@ -1299,7 +1302,8 @@ struct SortedNodes {
 };
 
 // Orders idx[0, m) so that consecutive runs of kTB nodes are compact boxes: recursive bisection
-// across the longest side, at a multiple of kTB nodes. A tile's own nodes stay in node order.
+// across the longest side, at a multiple of kTB nodes. A tile's own nodes stay in node order. Large
+// halves are tasks of the caller's thread team.
 void bisect_nodes(const double* pts, int32_t* idx, int64_t m) {
     if (m > kTB) {
         double lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
@@ -1317,6 +1321,7 @@ void bisect_nodes(const double* pts, int32_t* idx, int64_t m) {
             const double p = pts[3 * (int64_t)a + ax], q = pts[3 * (int64_t)b + ax];
             return p < q || (p == q && a < b);
         });
+#pragma omp task if (m > 8192)
         bisect_nodes(pts, idx, half);
         bisect_nodes(pts, idx + half, m - half);
     } else {
@@ -1380,9 +1385,18 @@ SortedNodes sort_nodes(const double* pts, const double* nrm, const double* w, in
         const bool in_plane = of[i] >= 0 && planes[of[i]].second >= kPlaneMin;
         so.perm[in_plane ? at[of[i]]++ : at.back()++] = (int32_t)i;
     }
-    for (size_t p = 0; p < planes.size(); ++p)
-        if (planes[p].second >= kPlaneMin) bisect_nodes(pts, &so.perm[at[p] - planes[p].second], planes[p].second);
-    if (rest > 0) bisect_nodes(pts, &so.perm[at.back() - rest], rest);
+#pragma omp parallel num_threads(8) if (n > 16384)
+#pragma omp single
+    {
+        for (size_t p = 0; p < planes.size(); ++p)
+            if (planes[p].second >= kPlaneMin) {
+                int32_t* idx = &so.perm[at[p] - planes[p].second];
+                const int64_t m = planes[p].second;
+#pragma omp task firstprivate(idx, m)
+                bisect_nodes(pts, idx, m);
+            }
+        if (rest > 0) bisect_nodes(pts, &so.perm[at.back() - rest], rest);
+    }
     int ex = 0;
     if (std::isfinite(ext) && ext > 0.0) std::frexp(ext, &ex);
     const double scale = std::ldexp(1.0, -std::max(-300, std::min(300, ex)));
@@ -1466,6 +1480,7 @@ bie_geom* geom_create(const double* pts, const double* nrm, const double* w, con
     g->geom_bytes = sizeof(double) * ((size_t)n * 8 + (size_t)g->ns * 4) + sizeof(int32_t) * (size_t)g->ns + (nblocks > 0 ? (sizeof(int32_t) * ((size_t)npanels + 1 + nblocks) +
                                                                      sizeof(double) * (size_t)nblocks * nb * nb)
                                                                   : 0);
+    ++g_geoms;
     return g.release();
 }
 
@@ -1541,6 +1556,7 @@ bool geom_trim_if_below(bie_geom* g, size_t free_floor) {
 void geom_trim_if_short(bie_geom* g) { geom_trim_if_below(g, 0); }
 
 void geom_destroy(bie_geom* g) {
+    if (--g_geoms == 0) copy_release();
     {
         DeviceGuard dg(g->device);
         if (g->stream) cudaStreamSynchronize(g->stream);
@@ -1631,7 +1647,7 @@ void matvec_host(bie_geom* g, const double* X, double* Y, int k, int precision, 
     g->io_a.ensure(sizeof(double) * nk);
     g->io_b.ensure(sizeof(double) * nk);
     g->xo.ensure(sizeof(double) * nk);
-    BIE_CK(cudaMemcpyAsync(g->io_a.p, X, sizeof(double) * nk, cudaMemcpyHostToDevice, s));
+    copy_in(g->io_a.p, X, sizeof(double) * nk, s);
     {
         Prof pf(g, BIE_KERNEL_OTHER, s);
         k_colmajor_to_nodemajor<<<grid1(nk), 256, 0, s>>>(g->io_a.as<double>(), g->n, k, g->io_b.as<double>());
@@ -1642,7 +1658,7 @@ void matvec_host(bie_geom* g, const double* X, double* Y, int k, int precision, 
         k_nodemajor_to_colmajor<<<grid1(nk), 256, 0, s>>>(g->xo.as<double>(), g->n, k, g->io_a.as<double>());
     }
     BIE_CK(cudaGetLastError());
-    BIE_CK(cudaMemcpyAsync(Y, g->io_a.p, sizeof(double) * nk, cudaMemcpyDeviceToHost, s));
+    copy_out(Y, g->io_a.p, sizeof(double) * nk, s);
     BIE_CK(cudaStreamSynchronize(s));
     check_device_error(g, s);
 }
@@ -1679,7 +1695,7 @@ void rhs_point_host(bie_geom* g, const double* src, const double* q, const doubl
         k_nodemajor_to_colmajor<<<grid1(nk), 256, 0, s>>>(g->io_b.as<double>(), g->n, k, g->io_a.as<double>());
     }
     BIE_CK(cudaGetLastError());
-    BIE_CK(cudaMemcpyAsync(F, g->io_a.p, sizeof(double) * nk, cudaMemcpyDeviceToHost, s));
+    copy_out(F, g->io_a.p, sizeof(double) * nk, s);
     BIE_CK(cudaStreamSynchronize(s));
 }
 
@@ -1704,7 +1720,7 @@ void potential_host(bie_geom* g, const double* S, int k, const double* T, int64_
     g->io_b.ensure(sizeof(double) * nk);
     g->xo.ensure(sizeof(double) * M * k);
     upload(g->small, T, (size_t)3 * M, s);
-    BIE_CK(cudaMemcpyAsync(g->io_a.p, S, sizeof(double) * nk, cudaMemcpyHostToDevice, s));
+    copy_in(g->io_a.p, S, sizeof(double) * nk, s);
     {
         Prof pf(g, BIE_KERNEL_OTHER, s);
         k_colmajor_to_nodemajor<<<grid1(nk), 256, 0, s>>>(g->io_a.as<double>(), g->n, k, g->io_b.as<double>());
@@ -1715,7 +1731,7 @@ void potential_host(bie_geom* g, const double* S, int k, const double* T, int64_
         k_nodemajor_to_colmajor<<<grid1(M * k), 256, 0, s>>>(g->xo.as<double>(), M, k, g->io_a.as<double>());
     }
     BIE_CK(cudaGetLastError());
-    BIE_CK(cudaMemcpyAsync(phi, g->io_a.p, sizeof(double) * M * k, cudaMemcpyDeviceToHost, s));
+    copy_out(phi, g->io_a.p, sizeof(double) * M * k, s);
     BIE_CK(cudaStreamSynchronize(s));
 }
 
@@ -1925,7 +1941,7 @@ int solve_point_host(bie_geom* g, const double* src, const double* q, const doub
         k_nodemajor_to_colmajor<<<grid1(nk), 256, 0, s>>>(g->sol.as<double>(), g->n, k, g->io_a.as<double>());
     }
     BIE_CK(cudaGetLastError());
-    BIE_CK(cudaMemcpyAsync(Sigma, g->io_a.p, sizeof(double) * nk, cudaMemcpyDeviceToHost, s));
+    copy_out(Sigma, g->io_a.p, sizeof(double) * nk, s);
     BIE_CK(cudaStreamSynchronize(s));
     geom_trim_if_short(g);
     return rc;
@@ -1938,7 +1954,7 @@ int solve_host(bie_geom* g, const double* F, double* Sigma, int k, const bie_sol
     g->io_a.ensure(sizeof(double) * nk);
     g->io_b.ensure(sizeof(double) * nk);
     g->sol.ensure(sizeof(double) * nk);  // output buffer, never aliased by the solver's scratch
-    BIE_CK(cudaMemcpyAsync(g->io_a.p, F, sizeof(double) * nk, cudaMemcpyHostToDevice, s));
+    copy_in(g->io_a.p, F, sizeof(double) * nk, s);
     {
         Prof pf(g, BIE_KERNEL_OTHER, s);
         k_colmajor_to_nodemajor<<<grid1(nk), 256, 0, s>>>(g->io_a.as<double>(), g->n, k, g->io_b.as<double>());
@@ -1949,7 +1965,7 @@ int solve_host(bie_geom* g, const double* F, double* Sigma, int k, const bie_sol
         k_nodemajor_to_colmajor<<<grid1(nk), 256, 0, s>>>(g->sol.as<double>(), g->n, k, g->io_a.as<double>());
     }
     BIE_CK(cudaGetLastError());
-    BIE_CK(cudaMemcpyAsync(Sigma, g->io_a.p, sizeof(double) * nk, cudaMemcpyDeviceToHost, s));
+    copy_out(Sigma, g->io_a.p, sizeof(double) * nk, s);
     BIE_CK(cudaStreamSynchronize(s));
     geom_trim_if_short(g);
     return rc;
@@ -2458,7 +2474,7 @@ int solve_group_point_host(bie_geom* const* gs, int G, const double* const* src,
         const int64_t nk = g->n * (int64_t)ks[i];
         k_nodemajor_to_colmajor<<<grid1(nk), 256, 0, s>>>(g->sol.as<double>(), g->n, ks[i], g->io_a.as<double>());
         BIE_CK(cudaGetLastError());
-        BIE_CK(cudaMemcpyAsync(Sigma[i], g->io_a.p, sizeof(double) * nk, cudaMemcpyDeviceToHost, s));
+        copy_out(Sigma[i], g->io_a.p, sizeof(double) * nk, s);
     }
     BIE_CK(cudaStreamSynchronize(s));
     for (int i = 0; i < G; ++i) geom_trim_if_short(gs[i]);

@@ -37,6 +37,13 @@ struct Buf {
     T* as() const { return (T*)p; }
 };
 
+// Copies between host arrays and the current device, ordered on s (hostcopy.cu). Large pageable arrays go
+// through a pinned buffer; copy_out's array is complete when the stream is (as with cudaMemcpyAsync).
+// copy_release frees the buffers kept between calls but one (4 MB), when the last geometry is gone.
+void copy_in(void* dev, const void* host, size_t bytes, cudaStream_t s);
+void copy_out(void* host, const void* dev, size_t bytes, cudaStream_t s);
+void copy_release();
+
 bie_geom* geom_create(const double* pts, const double* nrm, const double* w, const double* diag, int64_t n,
                       int32_t npanels, int32_t nb, const int32_t* rowptr, const int32_t* col, const double* val,
                       int64_t nblocks, int device);
