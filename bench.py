@@ -1085,7 +1085,7 @@ def main():
     roofline = None
     if tc.launches:
         per_launch_ms = tc.ms / (tc.launches / 2)  # pack + tensor-core kernel per column block
-        flops = 6.0 * tc.pair_cols / (tc.launches / 2)  # three bf16 MMAs (2 flops each) per pair and column
+        flops = 6.0 * tc.pair_cols / (tc.launches / 2)  # algorithmic: three bf16 products (2 flops each) per pair and column
         achieved = flops / (per_launch_ms * 1e-3) / 1e12
         roofline = {"kernel": "k_dt_tc (tcgen05 split-BF16 x3 block direct sum, incl. Q packing)", "bound": "tensor",
                     "achieved": achieved, "peak": bf16_peak, "unit": "TFLOP/s", "frac": achieved / bf16_peak,

@@ -44,8 +44,8 @@ typedef enum {
 typedef enum {
     BIE_FP64 = 0,   /* plain: FP64 end to end */
     BIE_FP32 = 1,   /* FP32 direct sum (FP64 tile partials), FP64 corrections/diag */
-    BIE_BF16X3 = 2, /* split-BF16 three-term tensor-core RHS contraction (FP32 sum for k = 1, 2, 4),
-                       FP32 kernel tiles, FP64 corrections/diag */
+    BIE_BF16X3 = 2, /* split-BF16 (two pieces per operand) tensor-core RHS contraction (FP32 sum for
+                       k = 1, 2, 4), FP32 kernel tiles, FP64 corrections/diag */
     BIE_BF16X6 = 3  /* three bf16 pieces per operand, six tensor-core products (idem):
                        about FP32 accuracy; the refinement's residual updates use it */
 } bie_precision;
@@ -159,7 +159,10 @@ void bie_geom_destroy(bie_geom* g);
  * (dense, src/solver/dielectric_box3d.jl:1-17) and of
  * lhs_dielectric_box3d_fmm3d_corrected / BatchedDielectricOperator mul!
  * (src/solver/dielectric_box3d.jl:48-92, src/solver/multi_rhs.jl:103-136) with the
- * FMM replaced by the exact direct sum (j != i). Host arrays, N x k column-major. */
+ * FMM replaced by the exact direct sum (j != i). Host arrays, N x k column-major.
+ * Pairs whose kernel value is exactly zero because source and target lie in the same
+ * axis-aligned plane are not summed: a value that is not finite in X[j] reaches the rows
+ * of other planes, not those of node j's own (its corrections and diagonal aside). */
 int bie_matvec(bie_geom* g, const double* X, double* Y, int32_t k, int32_t precision, uint32_t flags);
 /* Same on device arrays (node-major N x k) ordered on `stream` (NULL = the handle's). */
 int bie_matvec_device(bie_geom* g, const double* dX, double* dY, int32_t k, int32_t precision, uint32_t flags,
@@ -343,7 +346,7 @@ int bie_profile_read(bie_geom* g, int kind, bie_kernel_time* out);
 /* Autotuned launch configuration of a direct-sum family on this geometry: family 0 =
  * tensor-core block sum (columns = min(k, 128), pieces 2 or 3), 1 = FP64 tensor-core
  * sum (columns = min(k, 64), pieces 0). The library times a few candidate launch
- * shapes (CTA shape, source split count) on the first application of each family and
+ * shapes (source split counts) on the first application of each family and
  * kernel instance (widths rounded up to a multiple of 16 for family 0, to 8, 16, 32 or 64
  * for family 1, so every width of an instance reads the same entry) and keeps the
  * fastest (environment variable BIE_NO_AUTOTUNE turns this
