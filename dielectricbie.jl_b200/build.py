@@ -21,7 +21,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 CU_SOURCES = ["bie_b200.cu", "solver.cu", "blocktc.cu", "dt64mma.cu", "noalloc.cu", "server.cu", "near_gpu.cu", "peaks.cu", "combine_bulk.cu", "combine_direct.cu", "hostcopy.cu", "probe.cu"]
-CPP_SOURCES = ["host_setup.cpp", "probe_setup.cpp"]
+CPP_SOURCES = ["host_setup.cpp", "probe_setup.cpp", "sorted_nodes.cpp"]
 
 
 def _nvcc() -> str:

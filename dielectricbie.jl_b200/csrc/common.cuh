@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sorted_nodes.h"
+
 namespace bie {
 
 // Packed FP32 pairs (sm_100 f32x2 arithmetic): one instruction applies the same
@@ -36,7 +38,6 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 
 
 constexpr double kInv4Pi = 0.079577471545947667884;  // 1 / (4 pi)
-constexpr int kTB = 128;  // targets per CTA of the direct-sum kernels (one per thread)
 constexpr int kTS = 128;  // sources per shared-memory tile
 
 // MUFU reciprocal square root (approximate, flush-to-zero): a single instruction.
@@ -45,17 +46,6 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
-
-// Tiles of kTB consecutive slots of the sorted node order (GeomDev). A planar tile's nodes
-// share one plane x_axis = const with normals +-e_axis, and that plane's nodes are the slots
-// [s0, s1): the kernel n_x . (x - y) / |x - y|^3 of such a target and such a source is exactly
-// zero, so the direct sums leave those slots out. axis = 3, s0 = s1 = 0: any other tile. o: the
-// middle of the tile's bounding box (the plane itself along a planar tile's axis), the origin
-// that the FP32 sums round coordinates relative to.
-struct TileInfo {
-    int32_t axis, s0, s1;
-    double o[3];
-};
 
 // Device-resident geometry: SoA FP64 arrays of length n in the caller's node order, and the
 // sorted order of the direct sums. Sorted order: the nodes of each coordinate plane with at
@@ -74,9 +64,6 @@ struct GeomDev {
     const TileInfo* tiles;            // one per kTB slots; null: no planar tile
     int64_t ns;                       // slots
 };
-constexpr double kFar = 1.0e18;
-constexpr int kPlaneMin = 256;
-
 // Slots a tile sums over (all but its own plane's) and the l-th of them (s0, s1 and l are
 // multiples of every source tile, so a source tile never straddles the gap).
 __device__ __forceinline__ int64_t live_slots(const GeomDev& g, const TileInfo& t) { return g.ns - (t.s1 - t.s0); }
