@@ -74,6 +74,30 @@ __device__ __forceinline__ int64_t live_chunk(int64_t live, int nsplit) {
     return (c + kTS - 1) / kTS * kTS;
 }
 
+// Near tiles of the FP32 sum (K2). A coordinate relative to the target tile's origin, rounded to FP32,
+// is off by up to 2^-25 of the tile's half side h, which at a distance r puts an error of a few
+// 2^-25 h / r into a kernel value: below that of the FP32 operations unless the tiles (nearly) touch.
+// For source tiles closer than h / 4 the differences are therefore formed from two FP32 numbers a
+// coordinate (the rounded one and what it leaves), which makes them good to an FP32 rounding.
+// 23,040 nodes, random values: 1.2 % of the tile pairs, error of the FP32 sum 1.3e-6 -> 1.9e-7.
+struct NearBox {
+    double o[3], reach[3];
+    __device__ __forceinline__ explicit NearBox(const TileInfo& t) {
+        const double gap = 0.25 * fmax(t.h[0], fmax(t.h[1], t.h[2]));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            o[c] = t.o[c];
+            reach[c] = t.h[c] + gap;
+        }
+    }
+    __device__ __forceinline__ bool holds(const TileInfo& s) const {
+        return fabs(s.o[0] - o[0]) - s.h[0] < reach[0] && fabs(s.o[1] - o[1]) - s.h[1] < reach[1] &&
+               fabs(s.o[2] - o[2]) - s.h[2] < reach[2];
+    }
+};
+// What the FP32 rounding f of x leaves.
+__device__ __forceinline__ float rest32(double x, float f) { return (float)(x - (double)f); }
+
 // FP64 seed of 1 / sqrt(x), relative error about 2^-20: one MUFU instruction (PTX
 // rsqrt.approx.ftz.f64).
 __device__ __forceinline__ double rsqrt_seed(double x) {

@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(NTHR, occ<NC>()) k_dt_f64_mma(GeomDev g, const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int grp = lane >> 2, kq = lane & 3;
     const int64_t t0 = (int64_t)blockIdx.x * TB;
-    const TileInfo ti = !POT && g.tiles ? g.tiles[t0 / kTB] : TileInfo{3, 0, 0, {0.0, 0.0, 0.0}};
+    const TileInfo ti = !POT && g.tiles ? g.tiles[t0 / kTB] : TileInfo{3, 0, 0, {}, {}};
     // coordinate arrays, the tile's axis first
     const double* pa = ti.axis == 1 ? g.sy : (ti.axis == 2 ? g.sz : g.sx);
     const double* pb = ti.axis == 1 ? g.sz : (ti.axis == 2 ? g.sx : g.sy);

@@ -10,6 +10,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "arnoldi.cuh"
 #include "common.cuh"
@@ -37,7 +38,7 @@ __global__ void __launch_bounds__(kTB) k_dt_f64(GeomDev g, const double* __restr
     double* s1 = s0 + kTS;  // planar: the other two coordinates; else y, z
     double* s2 = s1 + kTS;
     double* sq = s2 + kTS;  // [kTS][C]
-    const TileInfo ti = g.tiles ? g.tiles[blockIdx.x] : TileInfo{3, 0, 0, {0.0, 0.0, 0.0}};
+    const TileInfo ti = g.tiles ? g.tiles[blockIdx.x] : TileInfo{3, 0, 0, {}, {}};
     const bool planar = ti.axis < 3;
     const int64_t t0 = (int64_t)blockIdx.x * kTB;
     const int64_t slot = t0 + threadIdx.x;
@@ -119,15 +120,18 @@ __global__ void __launch_bounds__(kTB) k_dt_f64(GeomDev g, const double* __restr
 
 // ---------------------------------------------------------------------------
 // K2: FP32 direct D^T sum with FP64 tile partials ("refined" inner operator).
-// Coordinates are rounded to FP32 relative to the middle of the target tile (keeps near-pair
-// differences accurate), rsqrt runs on the MUFU pipe, each shared-memory tile accumulates in
-// FP32 and is folded into FP64.
+// Coordinates are rounded to FP32 relative to the middle of the target tile. Up to 4 columns, the
+// widths that the solvers run here, near tiles (NearBox) take what the rounding leaves as well: 1
+// column at 2,560 nodes 9.8 -> 10.7 us, at 23,040 134 -> 137 us, 4 columns there 214 -> 226 us; more
+// columns, which only a caller's own product takes, leave it out.
+// rsqrt runs on the MUFU pipe, each shared-memory tile accumulates in FP32 and is folded into FP64.
 //
 // Bound by the FP32 pipe, then by the MUFU. Source pairs (t, t + 1) run as packed f32x2
 // operations. As in K1, a planar tile's difference along the axis and its square belong to the
 // source (7 operations and one MUFU a pair at C = 1, against 13 in other tiles), and sources of
 // the tile's own plane are left out.
 // ---------------------------------------------------------------------------
+template <int C> constexpr int f32_arrays() { return C <= 4 ? 6 : 3; }  // coordinate arrays of a staged tile
 template <int C>
 __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restrict__ X, int ldx, int c0,
                                                   const double* __restrict__ pre, double* __restrict__ part, int ldp) {
@@ -135,7 +139,10 @@ __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restr
     float* s0 = smf;        // planar: squared difference along the axis; else -x
     float* s1 = s0 + kTS;   // minus the other two coordinates; else -y, -z
     float* s2 = s1 + kTS;
-    float* sq = s2 + kTS;   // [C][kTS]: column c of the tile's sources, contiguous
+    float* e0 = s2 + kTS;   // near tiles, C <= 4: what the rounding of the coordinates leaves
+    float* e1 = e0 + kTS;
+    float* e2 = e1 + kTS;
+    float* sq = smf + f32_arrays<C>() * kTS;  // [C][kTS]: column c of the tile's sources, contiguous
     const TileInfo& ti = g.tiles[blockIdx.x];
     const int axis = ti.axis;
     const bool planar = axis < 3;
@@ -149,8 +156,10 @@ __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restr
     const double oa = ti.o[axis == 1 ? 1 : (axis == 2 ? 2 : 0)], ob = ti.o[axis == 1 ? 2 : (axis == 2 ? 0 : 1)],
                  oc = ti.o[axis == 1 ? 0 : (axis == 2 ? 1 : 2)];
     float xa = -1.0e18f, xb = -1.0e18f, xc = -1.0e18f, n0 = 0.f, n1 = 0.f, n2 = 0.f;
+    float ea = 0.f, eb = 0.f, ec = 0.f;
     if (valid) {
         xa = (float)(pa[slot] - oa); xb = (float)(pb[slot] - ob); xc = (float)(pc[slot] - oc);
+        ea = rest32(pa[slot] - oa, xa); eb = rest32(pb[slot] - ob, xb); ec = rest32(pc[slot] - oc, xc);
         n0 = (float)g.nx[i]; n1 = (float)g.ny[i]; n2 = (float)g.nz[i];
     }
     const uint64_t tA = pk2(xa, xa), tB = pk2(xb, xb), tCc = pk2(xc, xc);
@@ -161,55 +170,75 @@ __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restr
     for (int c = 0; c < C; ++c) acc[c] = 0.0;
     const int64_t live = live_slots(g, ti), chunk = live_chunk(live, gridDim.y);
     const int64_t l1 = min(live, ((int64_t)blockIdx.y + 1) * chunk);
+    uint32_t nears = 0;
+    int done = 0;
     for (int64_t l = (int64_t)blockIdx.y * chunk; l < l1; l += kTS) {
         const int64_t j = live_slot(ti, l) + threadIdx.x;  // slots come in whole tiles
         const int t = threadIdx.x;
+        if (f32_arrays<C>() == 6 && done % 32 == 0) {  // the next 32 tiles, one a lane
+            const NearBox box(ti);
+            const int64_t lm = l + (threadIdx.x & 31) * kTS;
+            nears = __ballot_sync(0xFFFFFFFFu, lm < l1 && box.holds(g.tiles[live_slot(ti, lm) / kTB]));
+        }
+        const bool near = nears >> (done++ & 31) & 1u;
         const double a = pa[j], b = pb[j], cc = pc[j];
         const int64_t p = g.perm[j];
         double wj = p >= 0 ? g.sw[j] * (pre ? pre[p] : 1.0) : 0.0;
         double xr[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) xr[c] = p >= 0 ? X[p * ldx + c0 + c] : 0.0;
-        float f0 = (float)(oa - a);
-        if (planar) {
-            wj *= oa - a;
-            f0 *= f0;
-        }
+        const float da = (float)(oa - a), db = (float)(ob - b), dc = (float)(oc - cc);
+        if (planar) wj *= oa - a;
         __syncthreads();
-        s0[t] = f0; s1[t] = (float)(ob - b); s2[t] = (float)(oc - cc);
+        s0[t] = planar ? da * da : da; s1[t] = db; s2[t] = dc;
+        if (near) {
+            e0[t] = rest32(oa - a, da); e1[t] = rest32(ob - b, db); e2[t] = rest32(oc - cc, dc);
+        }
 #pragma unroll
         for (int c = 0; c < C; ++c) sq[c * kTS + t] = (float)(wj * xr[c]);
         __syncthreads();
         uint64_t a2c[C];
 #pragma unroll
         for (int c = 0; c < C; ++c) a2c[c] = 0ull;
-        if (planar) {
+        auto pair = [](const float* v, int u) { return *reinterpret_cast<const uint64_t*>(v + u); };
+        auto planar_sum = [&](auto two) {
 #pragma unroll 4
             for (int u = 0; u < kTS; u += 2) {
-                const uint64_t db = add2(tB, *reinterpret_cast<const uint64_t*>(s1 + u));
-                const uint64_t dc = add2(tCc, *reinterpret_cast<const uint64_t*>(s2 + u));
-                const float2 r2 = upk2(fma2(db, db, fma2(dc, dc, *reinterpret_cast<const uint64_t*>(s0 + u))));
+                uint64_t db = add2(tB, pair(s1, u)), dc = add2(tCc, pair(s2, u));
+                if (two) {
+                    db = add2(db, add2(pk2(eb, eb), pair(e1, u)));
+                    dc = add2(dc, add2(pk2(ec, ec), pair(e2, u)));
+                }
+                const float2 r2 = upk2(fma2(db, db, fma2(dc, dc, pair(s0, u))));
                 const uint64_t ri = pk2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
                 const uint64_t gk = mul2(ri, mul2(ri, ri));
 #pragma unroll
-                for (int c = 0; c < C; ++c)
-                    a2c[c] = fma2(gk, *reinterpret_cast<const uint64_t*>(sq + c * kTS + u), a2c[c]);
+                for (int c = 0; c < C; ++c) a2c[c] = fma2(gk, pair(sq + c * kTS, u), a2c[c]);
             }
-        } else {
+        };
+        auto general_sum = [&](auto two) {
 #pragma unroll 4
             for (int u = 0; u < kTS; u += 2) {
-                const uint64_t dx = add2(tA, *reinterpret_cast<const uint64_t*>(s0 + u));
-                const uint64_t dy = add2(tB, *reinterpret_cast<const uint64_t*>(s1 + u));
-                const uint64_t dz = add2(tCc, *reinterpret_cast<const uint64_t*>(s2 + u));
+                uint64_t dx = add2(tA, pair(s0, u)), dy = add2(tB, pair(s1, u)), dz = add2(tCc, pair(s2, u));
+                if (two) {
+                    dx = add2(dx, add2(pk2(ea, ea), pair(e0, u)));
+                    dy = add2(dy, add2(pk2(eb, eb), pair(e1, u)));
+                    dz = add2(dz, add2(pk2(ec, ec), pair(e2, u)));
+                }
                 const float2 r2 = upk2(fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, tiny))));
                 const uint64_t ri = pk2(rsqrt_approx(r2.x), rsqrt_approx(r2.y));
                 const uint64_t nd = fma2(nA, dx, fma2(nB, dy, mul2(nC, dz)));
                 const uint64_t gk = mul2(mul2(nd, ri), mul2(ri, ri));
 #pragma unroll
-                for (int c = 0; c < C; ++c)
-                    a2c[c] = fma2(gk, *reinterpret_cast<const uint64_t*>(sq + c * kTS + u), a2c[c]);
+                for (int c = 0; c < C; ++c) a2c[c] = fma2(gk, pair(sq + c * kTS, u), a2c[c]);
             }
-        }
+        };
+        using yes = std::integral_constant<bool, true>;
+        using no = std::integral_constant<bool, false>;
+        if (planar)
+            near ? planar_sum(yes()) : planar_sum(no());
+        else
+            near ? general_sum(yes()) : general_sum(no());
 #pragma unroll
         for (int c = 0; c < C; ++c) {
             const float2 s2v = upk2(a2c[c]);

@@ -210,7 +210,7 @@ void* kern_ptr(Kern kind) {
 
 template <int C>
 size_t kern_smem(Kern kind) {
-    return (size_t)(3 + C) * kTS * (kind == Kern::DT32 ? sizeof(float) : sizeof(double));
+    return kTS * (kind == Kern::DT32 ? (f32_arrays<C>() + C) * sizeof(float) : (3 + C) * sizeof(double));
 }
 
 // occupancy (CTAs per SM) of one instantiation; also raises its dynamic smem limit

@@ -86,12 +86,12 @@ SortedNodes sort_nodes(const double* pts, const double* nrm, const double* w, in
     ns += padded(rest);
     SortedNodes so;
     so.perm.assign((size_t)ns, -1);
-    so.tiles.assign((size_t)(ns / kTB), TileInfo{3, 0, 0, {0.0, 0.0, 0.0}});
+    so.tiles.assign((size_t)(ns / kTB), TileInfo{3, 0, 0, {}, {}});
     for (size_t p = 0; p < planes.size(); ++p) {
         if (planes[p].second < kPlaneMin) continue;
         const int64_t s0 = at[p], s1 = s0 + padded(planes[p].second);
         for (int64_t t = s0 / kTB; t < s1 / kTB; ++t)
-            so.tiles[t] = TileInfo{planes[p].first, (int32_t)s0, (int32_t)s1, {0.0, 0.0, 0.0}};
+            so.tiles[t] = TileInfo{planes[p].first, (int32_t)s0, (int32_t)s1, {}, {}};
     }
     for (int64_t i = 0; i < n; ++i) {
         const bool in_plane = of[i] >= 0 && planes[of[i]].second >= kPlaneMin;
@@ -127,6 +127,7 @@ SortedNodes sort_nodes(const double* pts, const double* nrm, const double* w, in
                 b = std::max(b, so.v[c][e]);
             }
             so.tiles[t].o[c] = a == b ? a : 0.5 * (a + b);  // exactly the plane's along its axis
+            so.tiles[t].h[c] = 0.5 * (b - a);
         }
     return so;
 }

@@ -12,12 +12,12 @@ constexpr double kFar = 1.0e18;  // coordinates of padding slots
 // Tiles of kTB consecutive slots of the sorted node order (GeomDev). A planar tile's nodes
 // share one plane x_axis = const with normals +-e_axis, and that plane's nodes are the slots
 // [s0, s1): the kernel n_x . (x - y) / |x - y|^3 of such a target and such a source is exactly
-// zero, so the direct sums leave those slots out. axis = 3, s0 = s1 = 0: any other tile. o: the
-// middle of the tile's bounding box (the plane itself along a planar tile's axis), the origin
-// that the FP32 sums round coordinates relative to.
+// zero, so the direct sums leave those slots out. axis = 3, s0 = s1 = 0: any other tile. o and h:
+// middle and half sides of the tile's bounding box (o is the plane itself along a planar tile's
+// axis); o is the origin that the FP32 sums take coordinates relative to.
 struct TileInfo {
     int32_t axis, s0, s1;
-    double o[3];
+    double o[3], h[3];
 };
 
 // The sorted order of the direct sums (GeomDev): scaled positions and weights, the node of each
