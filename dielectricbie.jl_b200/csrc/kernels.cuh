@@ -164,7 +164,10 @@ __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restr
     }
     const uint64_t tA = pk2(xa, xa), tB = pk2(xb, xb), tCc = pk2(xc, xc);
     const uint64_t nA = pk2(n0, n0), nB = pk2(n1, n1), nC = pk2(n2, n2);
-    const uint64_t tiny = pk2(1e-24f, 1e-24f);  // keeps the self pair's r^-3 finite: it contributes 0
+    // added to r^2: keeps r^-3 finite for the self pair, which contributes 0, and for nodes that face each
+    // other across less than 1e-13 of the geometry's extent
+    const float tiny1 = 1e-24f;
+    const uint64_t tiny = pk2(tiny1, tiny1);
     double acc[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) acc[c] = 0.0;
@@ -190,7 +193,7 @@ __global__ void __launch_bounds__(kTB) k_dt_f32(GeomDev g, const double* __restr
         const float da = (float)(oa - a), db = (float)(ob - b), dc = (float)(oc - cc);
         if (planar) wj *= oa - a;
         __syncthreads();
-        s0[t] = planar ? da * da : da; s1[t] = db; s2[t] = dc;
+        s0[t] = planar ? fmaf(da, da, tiny1) : da; s1[t] = db; s2[t] = dc;
         if (near) {
             e0[t] = rest32(oa - a, da); e1[t] = rest32(ob - b, db); e2[t] = rest32(oc - cc, dc);
         }

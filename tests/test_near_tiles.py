@@ -68,3 +68,29 @@ def test_edges_of_a_box_in_fp32(bie, rng, box):
     Y, _ = dense_apply(itf, X)
     got = op.mul(np.asfortranarray(X), precision="fp32", flags=2)
     assert np.linalg.norm(got - Y) / np.linalg.norm(Y) < 3.6e-7
+
+
+def sheets(bie, gap):
+    """Two parallel unit squares with the same panels, normals towards each other."""
+    x, w = bie.gausslegendre(4)
+    at = lambda i, j, z: np.array([i / 8, j / 8, z])
+    return bie.DielectricInterface([bie.rect_panel3d_discretize(at(i, j, z), at(i + 1, j, z), at(i + 1, j + 1, z),
+                                                                at(i, j + 1, z), x, w, (0.0, 0.0, n))
+                                    for z, n in ((0.0, 1.0), (gap, -1.0)) for i in range(8) for j in range(8)], 4.0, 1.0)
+
+
+@pytest.mark.parametrize("precision", ["fp32", "bf16x3", "bf16x6"])
+@pytest.mark.parametrize("bits", [30, 45, 50])
+def test_facing_nodes_almost_in_one_plane(bie, rng, bits, precision):
+    """Facing nodes 2^-bits apart: their term is the sum. r^2 + 1e-24 costs a relative 1.5e-24 / 4^-30, 2^-19,
+    at 2^-30; closer than the FP32 range holds, every result is still a number."""
+    itf = sheets(bie, 2.0 ** -bits)
+    op = bie.lhs_dielectric_box3d(itf)
+    X = rng.uniform(0.5, 1.5, (itf.n, 8))
+    for k in (1, 2, 3, 4, 8):
+        got = op.mul(np.asfortranarray(X[:, :k]), precision=precision, flags=2)  # without the diagonal
+        assert np.all(np.isfinite(got)), k
+        if bits == 30:
+            other = np.roll(np.arange(itf.n), itf.n // 2)
+            want = -(itf.weights[:, None] * X[:, :k])[other] * 4.0 ** bits / (4 * np.pi)
+            assert np.max(np.abs(got / want - 1)) < (2.0 ** -15.8 if precision == "bf16x3" else 2.0 ** -16.9), k
