@@ -1321,40 +1321,42 @@ bie_geom* geom_create(const double* pts, const double* nrm, const double* w, con
     g->nblocks = nblocks;
     std::vector<double> col3((size_t)n);
     cudaStream_t s = g->stream;
+    auto put = [&](bie::Buf& b, const auto* src, size_t count) {
+        upload(b, src, count, s);
+        g->geom_bytes += sizeof(*src) * count;
+    };
     bie::Buf* xs[3] = {&g->x, &g->y, &g->z};
     bie::Buf* ns[3] = {&g->nx, &g->ny, &g->nz};
     for (int c = 0; c < 3; ++c) {
         for (int64_t i = 0; i < n; ++i) col3[i] = pts[3 * i + c];
-        upload(*xs[c], col3.data(), n, s);
+        put(*xs[c], col3.data(), n);
         BIE_CK(cudaStreamSynchronize(s));
         for (int64_t i = 0; i < n; ++i) col3[i] = nrm[3 * i + c];
-        upload(*ns[c], col3.data(), n, s);
+        put(*ns[c], col3.data(), n);
         BIE_CK(cudaStreamSynchronize(s));
     }
-    upload(g->w, w, n, s);
-    upload(g->diag, diag, n, s);
+    put(g->w, w, n);
+    put(g->diag, diag, n);
     {
         const SortedNodes so = sort_nodes(pts, nrm, w, n);
         g->ns = (int64_t)so.perm.size();
-        for (int c = 0; c < 4; ++c) upload(c == 0 ? g->sx : (c == 1 ? g->sy : (c == 2 ? g->sz : g->sw)), so.v[c].data(), g->ns, s);
-        upload(g->perm, so.perm.data(), g->ns, s);
-        upload(g->tiles, so.tiles.data(), so.tiles.size(), s);
+        bie::Buf* sorted[4] = {&g->sx, &g->sy, &g->sz, &g->sw};
+        for (int c = 0; c < 4; ++c) put(*sorted[c], so.v[c].data(), g->ns);
+        put(g->perm, so.perm.data(), g->ns);
+        put(g->tiles, so.tiles.data(), so.tiles.size());
         BIE_CK(cudaStreamSynchronize(s));
     }
     g->errflag.ensure(sizeof(int));
     BIE_CK(cudaMemsetAsync(g->errflag.p, 0, sizeof(int), s));
     for (int64_t i = 0; i < n; ++i) col3[i] = diag[i] != 0.0 ? 1.0 / diag[i] : 1.0;
-    upload(g->pinv, col3.data(), n, s);
+    put(g->pinv, col3.data(), n);
     if (nblocks > 0) {
-        upload(g->rowptr, rowptr, (size_t)npanels + 1, s);
+        put(g->rowptr, rowptr, (size_t)npanels + 1);
         for (int32_t p = 0; p < npanels; ++p) g->max_row_blocks = std::max(g->max_row_blocks, rowptr[p + 1] - rowptr[p]);
-        upload(g->col, col, nblocks, s);
-        upload(g->val, val, (size_t)nblocks * nb * nb, s);
+        put(g->col, col, nblocks);
+        put(g->val, val, (size_t)nblocks * nb * nb);
     }
     BIE_CK(cudaStreamSynchronize(s));
-    g->geom_bytes = sizeof(double) * ((size_t)n * 8 + (size_t)g->ns * 4) + sizeof(int32_t) * (size_t)g->ns + (nblocks > 0 ? (sizeof(int32_t) * ((size_t)npanels + 1 + nblocks) +
-                                                                     sizeof(double) * (size_t)nblocks * nb * nb)
-                                                                  : 0);
     ++g_geoms;
     return g.release();
 }
