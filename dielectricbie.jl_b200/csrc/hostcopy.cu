@@ -2,9 +2,10 @@
 //
 // cudaMemcpyAsync moves pageable memory through the driver's own pinned buffer on the calling thread;
 // for a solve's result it also takes the page faults of an array that nobody has touched yet, one at a
-// time. Large copies go through a pinned buffer of this library instead, kThreads host threads each
-// with two slots of kPiece bytes: one slot is copied by the host while the other is on the link. The
-// host's share is bound by its memory bandwidth, so four threads, not all cores.
+// time. Large copies go through a pinned buffer of this library instead, up to kThreads host threads
+// (fewer where the caller's OpenMP setting says so) each with two slots of kPiece bytes: one slot is
+// copied by the host while the other is on the link. The host's share is bound by its memory
+// bandwidth, so four threads, not all cores.
 //
 // 21.5 MB (42,048 nodes x 64 columns), potentials at 1,000 probes, whole call: 2.1 -> 1.2 ms; the refined
 // solve's 21.5 MB into a fresh array: 38.9 -> 37.8 ms.
@@ -92,7 +93,7 @@ bool pageable(const void* p) {
 cudaError_t staged(bool in, char* dev, char* host, size_t bytes, Stage* st, cudaStream_t s) {
     const int64_t pieces = (int64_t)((bytes + kPiece - 1) / kPiece);
     std::atomic<int> err{(int)cudaSuccess};
-#pragma omp parallel num_threads(kThreads)
+#pragma omp parallel num_threads(std::min(kThreads, omp_get_max_threads()))
     {
         const int t = omp_get_thread_num(), nt = omp_get_num_threads();
         auto ck = [&](cudaError_t e) {

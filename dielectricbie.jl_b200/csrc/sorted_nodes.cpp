@@ -1,6 +1,8 @@
 // Sort of a geometry's nodes into the order of the direct sums.
 #include "sorted_nodes.h"
 
+#include <omp.h>
+
 #include <algorithm>
 #include <cmath>
 #include <map>
@@ -97,7 +99,8 @@ SortedNodes sort_nodes(const double* pts, const double* nrm, const double* w, in
         const bool in_plane = of[i] >= 0 && planes[of[i]].second >= kPlaneMin;
         so.perm[in_plane ? at[of[i]]++ : at.back()++] = (int32_t)i;
     }
-#pragma omp parallel num_threads(8) if (n > 16384)
+    // up to 8 threads, fewer where the caller's OpenMP setting says so
+#pragma omp parallel num_threads(std::min(8, omp_get_max_threads())) if (n > 16384)
 #pragma omp single
     {
         for (size_t p = 0; p < planes.size(); ++p)
