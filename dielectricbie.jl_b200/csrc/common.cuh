@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "sorted_nodes.h"
+#include "splits.h"
 
 namespace bie {
 
@@ -38,7 +39,6 @@ __device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
 
 
 constexpr double kInv4Pi = 0.079577471545947667884;  // 1 / (4 pi)
-constexpr int kTS = 128;  // sources per shared-memory tile
 
 // MUFU reciprocal square root (approximate, flush-to-zero): a single instruction.
 __device__ __forceinline__ float rsqrt_approx(float x) {

@@ -252,18 +252,33 @@ void launch(const GeomDev& g, const double* T, int64_t M, const double* X, int l
     k<<<grid, NTHR, smem<NC>(), s>>>(g, T, M, X, ldx, c0, kc, pre, part, ldp);
 }
 
+// Runs f(NC as an integral constant) for the instance of a pass of kc columns.
+template <class F>
+auto with_width(int kc, F&& f) {
+    using std::integral_constant;
+    if (kc > 32) return f(integral_constant<int, 64>());
+    if (kc > 16) return f(integral_constant<int, 32>());
+    if (kc > 8) return f(integral_constant<int, 16>());
+    return f(integral_constant<int, 8>());
+}
+
 template <bool POT>
 void launch_width(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc,
                   const double* pre, int nsplit, double* part, int ldp, cudaStream_t s) {
-    if (kc > 32)
-        launch<64, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    else if (kc > 16)
-        launch<32, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    else if (kc > 8)
-        launch<16, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
-    else
-        launch<8, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
+    with_width(kc, [&](auto nc) { launch<nc.value, POT>(g, T, M, X, ldx, c0, kc, pre, nsplit, part, ldp, s); });
     BIE_CK(cudaGetLastError());
+}
+
+// Targets per CTA and resident CTAs per SM of the instance of a pass of kc columns.
+struct Instance {
+    int tb, per_sm;
+};
+template <bool POT>
+Instance instance_of(int kc) {
+    return with_width(kc, [](auto nc) {
+        constexpr int NC = nc.value;
+        return Instance{32 * mtw<NC>(), occupancy((const void*)k_dt_f64_mma<NC, POT>, NTHR, smem<NC>())};
+    });
 }
 
 }  // namespace d64
@@ -275,19 +290,19 @@ void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int k
     d64::launch_width<false>(g, nullptr, 0, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
 }
 
-// Source splits of the potential at M targets: the largest number that one wave of CTAs holds.
+// Source splits of the potential at M targets, for the instance of the first pass. 20,000 targets, 42,048
+// nodes, at most one wave and now: 8 columns 1.78 and 1.41 ms, 17 columns 4.16 and 2.78, 64 columns
+// 6.27 and 4.50; 1,000 targets as before.
 int pot_f64_mma_splits(int64_t n, int64_t M, int k, int sms) {
-    const int kc = std::min(k, 64);
-    const int tb = 32 * (kc <= 16 ? d64::mtw<16>() : d64::mtw<64>()), per_sm = kc <= 32 ? d64::occ<32>() : d64::occ<64>();
-    const int64_t tiles = (M + tb - 1) / tb;
-    return (int)std::max<int64_t>(1, std::min<int64_t>((int64_t)sms * per_sm / tiles, (n + kTS - 1) / kTS));
+    const d64::Instance in = d64::instance_of<true>(std::min(k, 64));
+    return wave_splits(n, (M + in.tb - 1) / in.tb, (int64_t)sms * in.per_sm);
 }
 
 // Single-layer potential partials (laplace3d_pottrg, src/kernel/laplace3d.jl:69-82, without the
 // 1/(4 pi)) of columns [c0, c0 + kc), kc <= 64 and c0 a multiple of 64, at M targets T (3 x M):
 //   part[s][m][c0 + c] = sum_{j in split s} w_j X[j][c0 + c] / |x_m - y_j|
-// The same kernel with 1 / r for its value: 42,048 nodes, 1,000 targets, 64 columns 0.55 -> 0.27 ms with the split reduction, where
-// the sum on FP64 FMAs alone is limited by its shared-memory loads.
+// The same kernel with 1 / r for its value: 42,048 nodes, 1,000 targets, 64 columns 0.55 -> 0.27 ms with
+// the split reduction, where the sum on FP64 FMAs alone is limited by its shared-memory loads.
 void launch_pot_f64_mma(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc,
                         int nsplit, double* part, int ldp, cudaStream_t s) {
     GeomDev r = g;  // the nodes in the caller's order and unit: the targets are not scaled
