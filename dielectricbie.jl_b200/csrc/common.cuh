@@ -145,6 +145,7 @@ int tc_npad(int kc);
 // K1 with the FP64 tensor-core contraction (dt64mma.cu), columns [c0, c0 + kc), kc <= 64.
 void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int kc, const double* pre, int nsplit,
                        double* part, int ldp, cudaStream_t s);
+int dt_f64_mma_ctas_per_sm(int kc);  // of the instance for kc columns
 // Single-layer potential at M targets with the same contraction (dt64mma.cu).
 int pot_f64_mma_splits(int64_t n, int64_t M, int k, int sms);
 void launch_pot_f64_mma(const GeomDev& g, const double* T, int64_t M, const double* X, int ldx, int c0, int kc,

@@ -290,6 +290,8 @@ void launch_dt_f64_mma(const GeomDev& g, const double* X, int ldx, int c0, int k
     d64::launch_width<false>(g, nullptr, 0, X, ldx, c0, kc, pre, nsplit, part, ldp, s);
 }
 
+int dt_f64_mma_ctas_per_sm(int kc) { return d64::instance_of<false>(kc).per_sm; }
+
 // Source splits of the potential at M targets, for the instance of the first pass. 20,000 targets, 42,048
 // nodes, at most one wave and now: 8 columns 1.78 and 1.41 ms, 17 columns 4.16 and 2.78, 64 columns
 // 6.27 and 4.50; 1,000 targets as before.

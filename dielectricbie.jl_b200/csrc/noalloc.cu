@@ -111,8 +111,7 @@ void dt_apply_static(const double* x, const double* y, const double* z, const do
 
     // columns per group and source splits, so that nsplit * n * kc fits the scratch. The
     // split count follows the regular FP64 path's base rule (about four waves of 128-target
-    // tiles at two per SM); the kernel's CTAs hold 64 targets at three per SM, so this gives
-    // them about twice the splits of a matched wave model, which measured faster there
+    // tiles at two per SM, whatever the instance's own tile)
     const int kc = (int)std::min<int64_t>({64, (int64_t)k, kScratchDoubles / n});
     const int64_t tiles = (n + 127) / 128;
     const int64_t want = (int64_t)sms * 2 * 4;
