@@ -32,7 +32,7 @@ struct bie_geom {
     int64_t nblocks = 0;
     size_t geom_bytes = 0;
     bie::Buf x, y, z, nx, ny, nz, w, diag, pinv;
-    bie::Buf sx, sy, sz, sw, perm, tiles;  // sorted order of the direct sums (GeomDev)
+    bie::Buf sorted, perm, tiles;  // sorted order of the direct sums (GeomDev); sorted: x, y, z, w
     int64_t ns = 0;
     bie::Buf rowptr, col, val;
     // operator workspace
@@ -179,9 +179,10 @@ struct Prof {
 };
 
 GeomDev gdev(const bie_geom* g) {
+    const double* v = g->sorted.as<double>();
     return GeomDev{g->x.as<double>(), g->y.as<double>(), g->z.as<double>(), g->nx.as<double>(),
                    g->ny.as<double>(), g->nz.as<double>(), g->w.as<double>(), g->n,
-                   g->sx.as<double>(), g->sy.as<double>(), g->sz.as<double>(), g->sw.as<double>(),
+                   v, v + g->ns, v + 2 * g->ns, v + 3 * g->ns,
                    g->perm.as<int32_t>(), g->tiles.as<TileInfo>(), g->ns};
 }
 
@@ -1294,6 +1295,17 @@ namespace {
 
 std::atomic<int64_t> g_geoms{0};  // geometries alive
 
+// The sorted positions and weights (GeomDev) from those in the caller's order: v[c ns + slot].
+__global__ void k_sorted_nodes(GeomDev g, double scale, double* __restrict__ v) {
+    const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= g.ns) return;
+    const int64_t i = g.perm[t];
+    v[t] = i >= 0 ? g.x[i] * scale : kFar;
+    v[g.ns + t] = i >= 0 ? g.y[i] * scale : kFar;
+    v[2 * g.ns + t] = i >= 0 ? g.z[i] * scale : kFar;
+    v[3 * g.ns + t] = i >= 0 ? g.w[i] * scale * scale : 0.0;
+}
+
 }  // namespace
 
 bie_geom* geom_create(const double* pts, const double* nrm, const double* w, const double* diag, int64_t n,
@@ -1340,9 +1352,12 @@ bie_geom* geom_create(const double* pts, const double* nrm, const double* w, con
     {
         const SortedNodes so = sort_nodes(pts, nrm, w, n);
         g->ns = (int64_t)so.perm.size();
-        bie::Buf* sorted[4] = {&g->sx, &g->sy, &g->sz, &g->sw};
-        for (int c = 0; c < 4; ++c) put(*sorted[c], so.v[c].data(), g->ns);
         put(g->perm, so.perm.data(), g->ns);
+        const size_t bytes = sizeof(double) * 4 * (size_t)g->ns;
+        g->sorted.ensure(bytes);
+        g->geom_bytes += bytes;
+        k_sorted_nodes<<<grid1(g->ns), 256, 0, s>>>(gdev(g.get()), so.scale, g->sorted.as<double>());
+        BIE_CK(cudaGetLastError());
         put(g->tiles, so.tiles.data(), so.tiles.size());
         BIE_CK(cudaStreamSynchronize(s));
     }
@@ -1438,7 +1453,7 @@ void geom_destroy(bie_geom* g) {
         DeviceGuard dg(g->device);
         if (g->stream) cudaStreamSynchronize(g->stream);
         if (g->s_ls) cudaStreamSynchronize(g->s_ls);
-        bie::Buf* all[] = {&g->x, &g->y, &g->z, &g->nx, &g->ny, &g->nz, &g->w, &g->diag, &g->pinv, &g->sx, &g->sy, &g->sz, &g->sw,
+        bie::Buf* all[] = {&g->x, &g->y, &g->z, &g->nx, &g->ny, &g->nz, &g->w, &g->diag, &g->pinv, &g->sorted,
                            &g->perm, &g->tiles, &g->rowptr,
                            &g->col, &g->val, &g->part, &g->small, &g->bpack, &g->errflag, &g->cpart, &g->V, &g->W, &g->R, &g->gv, &g->cs, &g->sn,
                            &g->h, &g->h2, &g->hn, &g->beta, &g->eps, &g->active, &g->jlast, &g->yv, &g->resid,

@@ -20,15 +20,15 @@ struct TileInfo {
     double o[3], h[3];
 };
 
-// The sorted order of the direct sums (GeomDev): scaled positions and weights, the node of each
-// slot, and each tile's plane and origin.
+// The sorted order of the direct sums (GeomDev): the node of each slot, each tile's plane and origin, and
+// the power of two that the positions are scaled by.
 struct SortedNodes {
-    std::vector<double> v[4];  // x, y, z, w
     std::vector<int32_t> perm;
     std::vector<TileInfo> tiles;
+    double scale;
 };
 
-// Sorts n nodes (positions and normals 3 x n, weights).
+// Sorts n nodes (positions and normals 3 x n; the order does not depend on the weights).
 SortedNodes sort_nodes(const double* pts, const double* nrm, const double* w, int64_t n);
 
 }  // namespace bie
