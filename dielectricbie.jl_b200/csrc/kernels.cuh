@@ -13,6 +13,7 @@
 #include <type_traits>
 
 #include "arnoldi.cuh"
+#include "combine_tile.h"
 #include "common.cuh"
 
 namespace bie {
@@ -393,21 +394,6 @@ __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-
-// Slab row stride for a kt-column tile: kt rounded up to 8, plus 4 (stride = 4 or 12
-// mod 16 doubles, so a half-warp's fragment loads hit distinct banks).
-__host__ __device__ inline int comb_ldx(int kt) { return ((kt + 7) / 8) * 8 + 4; }
-
-// Shared memory of the block-row combine for nb-row panels, kt-column tiles and
-// `stages` pipeline stages (reused for the warps' final reduction).
-inline size_t combine_smem_bytes(int nb, int kt, int stages, int warps) {
-    const int mt = (nb + 7) / 8, kp = ((nb + 3) / 4) * 4;
-    const int ldc = mt * 8 + 4;
-    const size_t pipe = (size_t)stages * kp * (ldc + comb_ldx(kt) + 1);
-    const size_t red = (size_t)warps * mt * 2 * 32;  // cross-warp reduction of the accumulators
-    return sizeof(double) * std::max(pipe, red);
-}
 
 // With gsum != nullptr the panel's block list is split into groups of bpg blocks
 // (blockIdx.z = group) and each group writes its block sum to gsum[z][i][c]; the

@@ -505,21 +505,19 @@ void combine(bie_geom* g, const TP* part, int nsplit, const double* X, double* Y
     const int mt = (g->nb + 7) / 8;
     const bool panel_rows = g->nb > 0 && (int64_t)g->npanels * g->nb == g->n;
     // Loads straight into fragments for 16-node panels and, at 36 nodes, for up to 16 columns on few
-    // panels (more are HBM-bound: streaming form below) and for 17 to 24 columns on many (us a launch
-    // with the events around it, before and after: 160 panels of 16, 1 column 20.2 and 12.6, 64 columns
-    // 45.5 and 29.0; 640 panels of 36, 8 columns 31.1 and 22.6, but 1,168 panels 38.7 and 43.5; 19
-    // columns, 1,168 panels 70.6 and 58.8, but 96 panels 21.7 and 22.9)
-    const bool direct = g->nb == 16 || (g->nb == 36 && (k <= 16 ? g->npanels < 6 * g->sms : k <= 24 && g->npanels >= 4 * g->sms));
+    // panels (more are HBM-bound: streaming form below) and for 17 to 24 columns on many. us a launch
+    // with the events around it, before and after: 16 nodes, 160 panels, 1 column 20.2 and 12.6, 64
+    // columns 45.5 and 29.0, 2,632 panels, 64 columns 401 and 256, 128 columns 760 and 519; 36 nodes, 8
+    // columns, 640 panels 31.1 and 22.6, but 1,168 panels 38.7 and 43.5; 19 columns, 1,168 panels 70.6
+    // and 58.8, but 96 panels 21.7 and 22.9.
+    const bool direct = g->nb == 16 || (g->nb == 36 && (k <= 16 ? g->npanels < 6 * g->sms
+                                                                : k <= 24 && g->npanels >= 4 * g->sms));
     if (panel_rows && direct && !std::getenv("BIE_COMBINE_ROWS") &&
         launch_combine_direct<TP>(g->n, k, g->nb, g->npanels, part, nsplit, X, pre, dgp, rp, cl, vl, Y, s))
         return;
     if (panel_rows && mt <= 8) {
         // the block products on the FP64 tensor path, two pipeline stages
-        
-        // 64 columns a CTA read the blocks once instead of twice, at three CTAs per SM instead of four:
-        // 128 columns, 1,168 panels of 36: 197 us instead of 223; 64 columns: 126 instead of 121 there,
-        // 272 instead of 331 on 2,632 panels
-        const int ct = k > 64 || (k == 64 && g->npanels >= 12 * g->sms) ? 64 : 32;
+        const int ct = combine_tile(g->nb, k, g->npanels, g->sms);
         const size_t sm = combine_smem_bytes(g->nb, std::min(k, ct), 2, ct / 8);
         // narrow blocks of right-hand sides on meshes with enough block rows to fill the
         // GPU: the HBM-bound streaming form, where its layout conditions hold
