@@ -36,7 +36,7 @@
 // run one CTA per SM (NQ = 4, 512 columns).
 //
 // Measured, 42,048 nodes in two pieces, before and after: 8 columns 1.33 and 0.74 ms, 64 columns 1.50
-// and 0.82, 128 columns 2.19 and 1.16. 12.3 warp instructions per 32 pairs, where the arithmetic takes
+// and 0.82, 128 columns 2.19 and 1.16. 12.1 warp instructions per 32 pairs, where the arithmetic takes
 // 9 and the generator alone, without MMAs, runs 30 % faster.
 // Every mbarrier wait is bounded: on expiry the CTA records an error code and
 // returns after releasing its tensor memory.

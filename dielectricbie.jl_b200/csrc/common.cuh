@@ -106,8 +106,8 @@ __device__ __forceinline__ double rsqrt_seed(double x) {
     return y;
 }
 // 1 / r^3 from r2 = r^2. With the seed y and e = 1 - r2 y^2, 1 / r^3 = y^3 (1 - e)^(-3/2), the
-// binomial series cut after e^2: the next term, 35/16 e^3, is below 2^-56 for |e| < 2^-19.
-// 7 FP64 operations, where 1 / sqrt to full precision and its cube take about 11.
+// binomial series cut after e^2: the next term, 35/16 e^3, is below 2^-55 for |e| < 2^-19.
+// 6 FP64 operations, where 1 / sqrt to full precision and its cube take about 11.
 __device__ __forceinline__ double over_r3(double r2) {
     const double y = rsqrt_seed(r2);
     const double q = y * y;
